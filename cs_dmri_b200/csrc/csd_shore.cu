@@ -727,15 +727,15 @@ void ensure_sched(csd_handle* h, int64_t V) {
   h->schedCnt.ensure(kSchedSlotBytes * kSchedSlots);
 }
 
-template <int MT, int WARPS, bool G_IN_SMEM = true>
-void launch_fista_v3_t(csd_handle* h, const csd::FistaParams& p) {
+template <int MT, int WARPS, bool G_IN_SMEM, bool NONNEG>
+void launch_fista_v3_n(csd_handle* h, const csd::FistaParams& p) {
   constexpr int KP = 8 * MT;
   // Gram tiles (when staged) + per-warp y and b buffers
   const size_t smem = sizeof(double) * ((G_IN_SMEM ? 2 * static_cast<size_t>(MT) * MT * 32 : 0) + WARPS * 2 * KP * 8);
-  CSD_CUDA(cudaFuncSetAttribute(csd::k_fista_v3<MT, WARPS, G_IN_SMEM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  CSD_CUDA(cudaFuncSetAttribute(csd::k_fista_v3<MT, WARPS, G_IN_SMEM, NONNEG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(smem)));
   int per_sm = 0;
-  CSD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, csd::k_fista_v3<MT, WARPS, G_IN_SMEM>, 32 * WARPS, smem));
+  CSD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, csd::k_fista_v3<MT, WARPS, G_IN_SMEM, NONNEG>, 32 * WARPS, smem));
   per_sm = std::max(per_sm, 1);
   const int64_t warps_needed = (p.n_work + 7) / 8;
   const int sms = h->sm_cap > 0 ? std::min(h->sm_cap, h->num_sms) : h->num_sms;
@@ -746,7 +746,7 @@ void launch_fista_v3_t(csd_handle* h, const csd::FistaParams& p) {
   q.mom = h->mom.as<double>();
   cudaStream_t st = h->stream;
   if (!sched_enabled(h, p, blocks * WARPS * 8)) {
-    csd::k_fista_v3<MT, WARPS, G_IN_SMEM><<<static_cast<unsigned>(blocks), 32 * WARPS, smem, st>>>(q);
+    csd::k_fista_v3<MT, WARPS, G_IN_SMEM, NONNEG><<<static_cast<unsigned>(blocks), 32 * WARPS, smem, st>>>(q);
     CSD_LAUNCH();
     return;
   }
@@ -769,7 +769,7 @@ void launch_fista_v3_t(csd_handle* h, const csd::FistaParams& p) {
   q1.pend = pend;
   q1.pend_key = key;
   q1.n_pend = n_pend;
-  csd::k_fista_v3<MT, WARPS, G_IN_SMEM><<<static_cast<unsigned>(blocks), 32 * WARPS, smem, st>>>(q1);
+  csd::k_fista_v3<MT, WARPS, G_IN_SMEM, NONNEG><<<static_cast<unsigned>(blocks), 32 * WARPS, smem, st>>>(q1);
   CSD_LAUNCH();
   csd::k_sched_hist<<<h->num_sms, 256, 0, st>>>(key, n_pend, hist, p.iter_total ? p.iter_total + 2 : nullptr);
   CSD_LAUNCH();
@@ -783,8 +783,16 @@ void launch_fista_v3_t(csd_handle* h, const csd::FistaParams& p) {
   q2.n_work_dev = n_pend;
   q2.pend = nullptr;
   q2.pend_key = nullptr;
-  csd::k_fista_v3<MT, WARPS, G_IN_SMEM><<<static_cast<unsigned>(blocks), 32 * WARPS, smem, st>>>(q2);
+  csd::k_fista_v3<MT, WARPS, G_IN_SMEM, NONNEG><<<static_cast<unsigned>(blocks), 32 * WARPS, smem, st>>>(q2);
   CSD_LAUNCH();
+}
+
+template <int MT, int WARPS, bool G_IN_SMEM = true>
+void launch_fista_v3_t(csd_handle* h, const csd::FistaParams& p) {
+  if (p.non_negative)
+    launch_fista_v3_n<MT, WARPS, G_IN_SMEM, true>(h, p);
+  else
+    launch_fista_v3_n<MT, WARPS, G_IN_SMEM, false>(h, p);
 }
 
 // FISTA kernel variant: 0 = k_fista_fp64 (registers hold x, y, b); 3 / 4 =

@@ -224,6 +224,19 @@ struct FistaParams {
   const unsigned long long* n_work_dev; // work-list length on the device (nullptr: n_work)
 };
 
+// One entry of the proximal gradient step (src/solver/fista.rs:95-107), the
+// same in every FP64 FISTA kernel: the candidate y - step (G y - b) / n with c
+// = step / n, soft-thresholded by th = step alpha (0 inside and for NaN), and
+// projected when NONNEG.
+template <bool NONNEG>
+__device__ __forceinline__ double fista_prox(double gy, double b, double y, double c, double th) {
+  const double cand = fma(-c, __dsub_rn(gy, b), y);
+  const bool above = cand > th;
+  if (NONNEG) return above ? __dsub_rn(cand, th) : 0.0;
+  const double sv = __dsub_rn(cand, above ? th : -th);
+  return (above || cand < -th) ? sv : 0.0;
+}
+
 // One warp fits 8 voxels at a time (the 8 columns of an m8n8k4 tile).  Lane
 // l holds rows 8*mt + l/4 of voxel columns 2*(l%4) + {0,1} for every row tile
 // mt: the DMMA accumulator layout, so the elementwise FISTA update, the
@@ -255,6 +268,7 @@ __global__ void __launch_bounds__(256) k_fista_fp64(FistaParams p) {
   bool need[2] = {true, true};
   bool exhausted = false;
   unsigned long long executed = 0;  // voxel-iterations run by this warp
+  const double c = p.step * p.n_inv;
 
   while (true) {
     // ---- refill finished or empty slots from the queue (warp-aggregated)
@@ -341,18 +355,10 @@ __global__ void __launch_bounds__(256) k_fista_fp64(FistaParams p) {
     for (int mt = 0; mt < MT; ++mt) {
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
-        const double grad = __dmul_rn(__dsub_rn(acc[mt][j], b[mt][j]), p.n_inv);
-        const double cand = __dsub_rn(y[mt][j], __dmul_rn(p.step, grad));
-        double sv;
-        if (cand > thr[j])
-          sv = __dsub_rn(cand, thr[j]);
-        else if (cand < -thr[j])
-          sv = __dadd_rn(cand, thr[j]);
-        else
-          sv = 0.0;
-        const double xn = p.non_negative ? fmax(sv, 0.0) : sv;
+        const double xn = p.non_negative ? fista_prox<true>(acc[mt][j], b[mt][j], y[mt][j], c, thr[j])
+                                         : fista_prox<false>(acc[mt][j], b[mt][j], y[mt][j], c, thr[j]);
         const double d = __dsub_rn(xn, x[mt][j]);
-        y[mt][j] = __dadd_rn(xn, __dmul_rn(mom[j], d));
+        y[mt][j] = fma(mom[j], d, xn);
         dx2[j] = __dadd_rn(dx2[j], __dmul_rn(d, d));
         xn2[j] = __dadd_rn(xn2[j], __dmul_rn(xn, xn));
         x[mt][j] = xn;
@@ -399,9 +405,16 @@ __global__ void __launch_bounds__(256) k_fista_fp64(FistaParams p) {
 //    thread-private shared buffer, so registers hold just x and the
 //    accumulators and 12 warps fit per SM;
 //  * the k-step loop is outermost, so consecutive DMMAs update different
-//    accumulators (no dependent DMMA back to back), and a k-step whose y
-//    entries are exactly zero for all eight voxels is skipped (it would add
-//    only zeros): the iterates are sparse, so about half the DMMAs go;
+//    accumulators (no dependent DMMA back to back), and runs over the live
+//    k-steps only: one whose y entries are exactly zero for all eight voxels
+//    would add only zeros, and the iterates are sparse (52 % live at order 6).
+//    The update that writes y marks them, one bit a lane and row tile, and
+//    one OR over the warp makes the list: no vote or branch for a dead
+//    k-step;
+//  * one shared update of an entry (fista_prox) in ten FP64 operations, the
+//    projection compiled in or out; the FP64 pipe carries the DMMAs and this
+//    update, 47 + 11 of the 82 SM cycles a voxel-iteration takes at order 6
+//    (brain-sized volume of 299,432 voxels: 14.4 -> 12.4 ms a fit);
 //  * the momentum (t_k - 1) / t_{k+1} comes from a table: t_k depends only on
 //    the iteration index, and the host evaluates the same IEEE expressions;
 //  * the stopping test sqrt(dx2) / max(sqrt(xn2), 1e-12) < tol is evaluated
@@ -412,7 +425,7 @@ __global__ void __launch_bounds__(256) k_fista_fp64(FistaParams p) {
 //
 // G_IN_SMEM = false (large K, where the tiles would crowd out the warp
 // buffers): the tiles are read through the L1/L2 caches instead.
-template <int MT, int WARPS, bool G_IN_SMEM>
+template <int MT, int WARPS, bool G_IN_SMEM, bool NONNEG>
 __global__ void __launch_bounds__(32 * WARPS) k_fista_v3(FistaParams p) {
   constexpr int KP = 8 * MT, KT = 2 * MT;
   constexpr int G_WORDS = G_IN_SMEM ? MT * KT * 32 : 0;
@@ -433,14 +446,20 @@ __global__ void __launch_bounds__(32 * WARPS) k_fista_v3(FistaParams p) {
   double thr[2] = {p.thr, p.thr};
   bool need[2] = {true, true};
   bool exhausted = false;
-  unsigned long long executed = 0, ksteps = 0;
+  unsigned executed = 0, ksteps = 0;
   const double tol2x4 = 4.0 * p.tol * p.tol;
+  const double c = p.step * p.n_inv;
   float sl[2] = {0.f, 0.f}, skl[2] = {0.f, 0.f};  // pass 1: sums of log2(rel^2) and k log2(rel^2)
   const int w0 = p.cap - p.cap / 2;                 // window of the slope fit: iterations w0+1 .. cap
+  // k-steps with a non-zero y entry (a superset: the others are skipped), in words of 32
+  constexpr int LW = (KT + 31) / 32;
+  unsigned live[LW];
+#pragma unroll
+  for (int w = 0; w < LW; ++w) live[w] = kFull;
 
   while (true) {
     // ---- refill (warp-aggregated queue)
-    {
+    if (__any_sync(kFull, need[0] || need[1])) {
       const unsigned n0 = __ballot_sync(kFull, lane < 4 && need[0]);
       const unsigned n1 = __ballot_sync(kFull, lane < 4 && need[1]);
       unsigned colmask = 0;
@@ -449,6 +468,10 @@ __global__ void __launch_bounds__(32 * WARPS) k_fista_v3(FistaParams p) {
         colmask |= (((n0 >> l) & 1u) << (2 * l)) | (((n1 >> l) & 1u) << (2 * l + 1));
       const int nneed = __popc(colmask);
       if (nneed > 0) {
+        if (p.resume || p.warm) {  // slots may start from a non-zero point
+#pragma unroll
+          for (int w = 0; w < LW; ++w) live[w] = kFull;
+        }
         const unsigned long long V_END = p.n_work_dev ? *p.n_work_dev : static_cast<unsigned long long>(p.n_work);
         unsigned long long base = V_END;
         if (!exhausted) {
@@ -496,13 +519,16 @@ __global__ void __launch_bounds__(32 * WARPS) k_fista_v3(FistaParams p) {
     double acc[MT][2];
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt) acc[mt][0] = acc[mt][1] = 0.0;
+    // A k-step whose four y entries are exactly zero for all eight voxels adds
+    // only zeros (soft thresholding keeps most of y at 0): only the live ones run.
 #pragma unroll
-    for (int kt = 0; kt < KT; ++kt) {
-      const double bf = ybuf[(4 * kt + q) * 8 + g];
-      // A k-step whose four y entries are exactly zero for all eight voxels
-      // adds only zeros: skip it (soft thresholding keeps most of y at 0).
-      if (__any_sync(kFull, bf != 0.0)) {
-        ++ksteps;
+    for (int w = 0; w < LW; ++w) {
+      unsigned m = live[w] & (KT - 32 * w >= 32 ? kFull : (1u << (KT - 32 * w)) - 1u);
+      ksteps += __popc(m);
+#pragma unroll 1
+      for (; m != 0; m &= m - 1) {
+        const int kt = 32 * w + __ffs(static_cast<int>(m)) - 1;
+        const double bf = ybuf[(4 * kt + q) * 8 + g];
 #pragma unroll
         for (int mt = 0; mt < MT; ++mt) {
           const double af = G_IN_SMEM ? sG[(mt * KT + kt) * 32 + lane] : __ldg(sG + (mt * KT + kt) * 32 + lane);
@@ -517,6 +543,8 @@ __global__ void __launch_bounds__(32 * WARPS) k_fista_v3(FistaParams p) {
 #pragma unroll
     for (int j = 0; j < 2; ++j) mom[j] = (vid[j] >= 0) ? p.mom[it[j]] : 0.0;
 #pragma unroll
+    for (int w = 0; w < LW; ++w) live[w] = 0u;
+#pragma unroll
     for (int mt = 0; mt < MT; ++mt) {
       const int row = 8 * mt + g;
       const double2 yv = *reinterpret_cast<const double2*>(&ybuf[row * 8 + 2 * q]);
@@ -525,24 +553,19 @@ __global__ void __launch_bounds__(32 * WARPS) k_fista_v3(FistaParams p) {
       double yo[2];
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
-        const double grad = __dmul_rn(__dsub_rn(acc[mt][j], bb[j]), p.n_inv);
-        const double cand = __dsub_rn(yy[j], __dmul_rn(p.step, grad));
-        double sv;
-        if (cand > thr[j])
-          sv = __dsub_rn(cand, thr[j]);
-        else if (cand < -thr[j])
-          sv = __dadd_rn(cand, thr[j]);
-        else
-          sv = 0.0;
-        const double xn = p.non_negative ? fmax(sv, 0.0) : sv;
+        const double xn = fista_prox<NONNEG>(acc[mt][j], bb[j], yy[j], c, thr[j]);
         const double d = __dsub_rn(xn, x[mt][j]);
-        yo[j] = __dadd_rn(xn, __dmul_rn(mom[j], d));
+        yo[j] = fma(mom[j], d, xn);
         dx2[j] = fma(d, d, dx2[j]);
         xn2[j] = fma(xn, xn, xn2[j]);
         x[mt][j] = xn;
       }
       *reinterpret_cast<double2*>(&ybuf[row * 8 + 2 * q]) = make_double2(yo[0], yo[1]);
+      if ((__double_as_longlong(yo[0]) | __double_as_longlong(yo[1])) != 0) live[mt / 16] |= 1u << (2 * (mt % 16));
     }
+    // rows 8 mt .. 8 mt + 3 (lanes 0-15) are k-step 2 mt, the others 2 mt + 1
+#pragma unroll
+    for (int w = 0; w < LW; ++w) live[w] = __reduce_or_sync(kFull, live[w] << (g >> 2));
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
 #pragma unroll
@@ -610,9 +633,9 @@ __global__ void __launch_bounds__(32 * WARPS) k_fista_v3(FistaParams p) {
   }
   if (p.iter_total) {
     for (int o = 16; o > 0; o >>= 1) executed += __shfl_xor_sync(kFull, executed, o);
-    if (lane == 0) atomicAdd(p.iter_total, executed);
+    if (lane == 0) atomicAdd(p.iter_total, static_cast<unsigned long long>(executed));
   }
-  if (p.kstep_total && lane == 0) atomicAdd(p.kstep_total, ksteps);
+  if (p.kstep_total && lane == 0) atomicAdd(p.kstep_total, static_cast<unsigned long long>(ksteps));
 }
 
 // Order of the second pass of the two-pass FISTA schedule: the voxels that
