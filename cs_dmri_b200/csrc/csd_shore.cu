@@ -40,6 +40,7 @@
 #include "path_kernels.cuh"
 #include "setup_kernels.cuh"
 #include "solve_kernels.cuh"
+#include "sparse_kernels.cuh"
 #include "icls_kernels.cuh"
 #include "mixed_kernels.cuh"
 #include "tf32_kernels.cuh"
@@ -727,15 +728,15 @@ void ensure_sched(csd_handle* h, int64_t V) {
   h->schedCnt.ensure(kSchedSlotBytes * kSchedSlots);
 }
 
-template <int MT, int WARPS, bool G_IN_SMEM, bool NONNEG>
+template <int MT, int WARPS, bool NONNEG>
 void launch_fista_v3_n(csd_handle* h, const csd::FistaParams& p) {
   constexpr int KP = 8 * MT;
-  // Gram tiles (when staged) + per-warp y and b buffers
-  const size_t smem = sizeof(double) * ((G_IN_SMEM ? 2 * static_cast<size_t>(MT) * MT * 32 : 0) + WARPS * 2 * KP * 8);
-  CSD_CUDA(cudaFuncSetAttribute(csd::k_fista_v3<MT, WARPS, G_IN_SMEM, NONNEG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  // Gram tiles + per-warp y and b buffers
+  const size_t smem = sizeof(double) * (2 * static_cast<size_t>(MT) * MT * 32 + WARPS * 2 * KP * 8);
+  CSD_CUDA(cudaFuncSetAttribute(csd::k_fista_v3<MT, WARPS, NONNEG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(smem)));
   int per_sm = 0;
-  CSD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, csd::k_fista_v3<MT, WARPS, G_IN_SMEM, NONNEG>, 32 * WARPS, smem));
+  CSD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, csd::k_fista_v3<MT, WARPS, NONNEG>, 32 * WARPS, smem));
   per_sm = std::max(per_sm, 1);
   const int64_t warps_needed = (p.n_work + 7) / 8;
   const int sms = h->sm_cap > 0 ? std::min(h->sm_cap, h->num_sms) : h->num_sms;
@@ -746,7 +747,7 @@ void launch_fista_v3_n(csd_handle* h, const csd::FistaParams& p) {
   q.mom = h->mom.as<double>();
   cudaStream_t st = h->stream;
   if (!sched_enabled(h, p, blocks * WARPS * 8)) {
-    csd::k_fista_v3<MT, WARPS, G_IN_SMEM, NONNEG><<<static_cast<unsigned>(blocks), 32 * WARPS, smem, st>>>(q);
+    csd::k_fista_v3<MT, WARPS, NONNEG><<<static_cast<unsigned>(blocks), 32 * WARPS, smem, st>>>(q);
     CSD_LAUNCH();
     return;
   }
@@ -769,7 +770,7 @@ void launch_fista_v3_n(csd_handle* h, const csd::FistaParams& p) {
   q1.pend = pend;
   q1.pend_key = key;
   q1.n_pend = n_pend;
-  csd::k_fista_v3<MT, WARPS, G_IN_SMEM, NONNEG><<<static_cast<unsigned>(blocks), 32 * WARPS, smem, st>>>(q1);
+  csd::k_fista_v3<MT, WARPS, NONNEG><<<static_cast<unsigned>(blocks), 32 * WARPS, smem, st>>>(q1);
   CSD_LAUNCH();
   csd::k_sched_hist<<<h->num_sms, 256, 0, st>>>(key, n_pend, hist, p.iter_total ? p.iter_total + 2 : nullptr);
   CSD_LAUNCH();
@@ -783,16 +784,89 @@ void launch_fista_v3_n(csd_handle* h, const csd::FistaParams& p) {
   q2.n_work_dev = n_pend;
   q2.pend = nullptr;
   q2.pend_key = nullptr;
-  csd::k_fista_v3<MT, WARPS, G_IN_SMEM, NONNEG><<<static_cast<unsigned>(blocks), 32 * WARPS, smem, st>>>(q2);
+  csd::k_fista_v3<MT, WARPS, NONNEG><<<static_cast<unsigned>(blocks), 32 * WARPS, smem, st>>>(q2);
   CSD_LAUNCH();
 }
 
-template <int MT, int WARPS, bool G_IN_SMEM = true>
+template <int MT, int WARPS>
 void launch_fista_v3_t(csd_handle* h, const csd::FistaParams& p) {
   if (p.non_negative)
-    launch_fista_v3_n<MT, WARPS, G_IN_SMEM, true>(h, p);
+    launch_fista_v3_n<MT, WARPS, true>(h, p);
   else
-    launch_fista_v3_n<MT, WARPS, G_IN_SMEM, false>(h, p);
+    launch_fista_v3_n<MT, WARPS, false>(h, p);
+}
+
+// k_fista_sparse over the work list of p: warps per CTA so that a short list
+// spreads over the SMs (at least four, which stage G).
+template <int K, int P, int MAXWARPS, int MINCTAS, bool NONNEG>
+void launch_fista_sparse_t(csd_handle* h, const csd::FistaParams& p) {
+  using S = csd::SparseShape<K, P>;
+  const int sms = h->sm_cap > 0 ? std::min(h->sm_cap, h->num_sms) : h->num_sms;
+  const int64_t need = (p.n_work + P - 1) / P;  // warps with a voxel in every slot
+  const int warps = static_cast<int>(std::min<int64_t>(MAXWARPS, std::max<int64_t>(4, (need + sms - 1) / sms)));
+  const size_t smem = S::G_BYTES + static_cast<size_t>(warps) * S::WARP_BYTES;
+  auto* kern = csd::k_fista_sparse<K, P, MAXWARPS, MINCTAS, NONNEG>;
+  CSD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  const int64_t blocks = std::max<int64_t>(
+      1, std::min<int64_t>(static_cast<int64_t>(sms) * MINCTAS, (need + warps - 1) / warps));
+  csd::FistaParams q = p;
+  q.G = h->G.as<double>();
+  q.mom = h->mom.as<double>();
+  kern<<<static_cast<unsigned>(blocks), 32 * warps, smem, h->stream>>>(q);
+  CSD_LAUNCH();
+}
+
+template <int K, int P, int MAXWARPS, int MINCTAS>
+void launch_fista_sparse_p(csd_handle* h, const csd::FistaParams& p) {
+  if (p.non_negative)
+    launch_fista_sparse_t<K, P, MAXWARPS, MINCTAS, true>(h, p);
+  else
+    launch_fista_sparse_t<K, P, MAXWARPS, MINCTAS, false>(h, p);
+}
+
+// Whether a fit of n_work voxels takes the sparse kernel (handle option
+// CSD_OPT_FISTA_SHAPE left at 0; every kernel computes the same iterates).
+// Measured per volume fit on B200, sparse against k_fista_v3, N = 259:
+//   order 4:   74,088 voxels 1.85 / 1.94 ms, 300,763 voxels 6.41 / 5.25 ms
+//   order 6:    4,000 voxels 0.99 / 2.80 ms, 74,088 voxels 4.29 / 4.32 ms,
+//             125,000 voxels 6.97 / 6.25 ms
+//   order 8:   32,000 voxels 4.56 / 6.87 ms, 300,763 voxels 33.2 / 47.5 ms
+// A warp of k_fista_v3 takes 2 us an iteration for its eight voxels and the
+// slowest voxel's up to 1,000 iterations set a small fit's time; a sparse warp
+// takes 0.3 us.  From four waves of slots the DMMA kernel's two-pass schedule
+// hides that tail and its throughput decides - except at order 8, where G's
+// tiles do not fit in shared memory beside the slots' vectors and 9 % of y's
+// entries are non-zero.
+bool sparse_fista(const csd_handle* h, int64_t n_work) {
+  if (h->K == 145) return true;
+  if (h->opt_shape != 0 || (h->K != 29 && h->K != 72)) return false;
+  return n_work < kSchedMinWaves * h->num_sms * 16 * 8;
+}
+
+// One voxel per warp has the shorter iteration, two share the reads of G's
+// columns (per voxel-iteration 85 against 72 wavefronts at order 6): two from
+// about twice the voxels that one per warp holds at once (order 6: 4,000
+// voxels 0.99 / 1.06 ms, 16,384 voxels 1.57 / 1.54 ms, 64,000 voxels 4.07 /
+// 3.77 ms; order 8: 8,000 voxels 1.56 / 1.80 ms, 16,000 voxels 2.43 / 2.40
+// ms).  At order 4 one is faster at every size measured (64,000 voxels 1.69 /
+// 1.78 ms).
+void launch_fista_sparse(csd_handle* h, const csd::FistaParams& p) {
+  switch (h->K) {
+    case 29: launch_fista_sparse_p<29, 1, 16, 2>(h, p); break;
+    case 72:
+      if (p.n_work > 64 * h->num_sms)
+        launch_fista_sparse_p<72, 2, 16, 1>(h, p);
+      else
+        launch_fista_sparse_p<72, 1, 16, 2>(h, p);
+      break;
+    case 145:
+      if (p.n_work > 96 * h->num_sms)
+        launch_fista_sparse_p<145, 2, 12, 1>(h, p);
+      else
+        launch_fista_sparse_p<145, 1, 16, 1>(h, p);
+      break;
+    default: throw Error{CSD_ERR_INVALID, "the sparse FISTA kernel is built for radial orders 4, 6 and 8"};
+  }
 }
 
 // FISTA kernel variant: 0 = k_fista_fp64 (registers hold x, y, b); 3 / 4 =
@@ -1257,6 +1331,10 @@ void launch_fista(csd_handle* h, int MT, const csd::FistaParams& p) {
     CSD_LAUNCH();
     return;
   }
+  if (sparse_fista(h, p.n_work)) {
+    launch_fista_sparse(h, p);
+    return;
+  }
   const int variant = fista_variant(h);
   if (variant == 3 || variant == 4) {
     switch (MT * 8 + variant) {
@@ -1268,10 +1346,6 @@ void launch_fista(csd_handle* h, int MT, const csd::FistaParams& p) {
       case 9 * 8 + 4: launch_fista_v3_t<9, 16>(h, p); return;
       default: break;
     }
-  }
-  if (MT == 19) {  // radial order 8 (K = 145): Gram tiles through the caches
-    launch_fista_v3_t<19, 8, false>(h, p);
-    return;
   }
   switch (MT) {
     case 1: launch_fista_t<1>(h, p); break;
@@ -1378,11 +1452,12 @@ void launch_resid_dmma_t(csd_handle* h, const csd::ResidParams& r) {
 // explicit per-voxel output (resid_out); a scatter of coefficients alone
 // (diagnostics off) skips them.
 void launch_epilogue(csd_handle* h, const csd::EpilogueParams& p) {
-  if (!h->dmma_resid || p.n_work == 0) {
-    if (p.n_work > 0) launch_epilogue_ffma(h, p);
+  if (p.n_work == 0) return;
+  const bool need_resid = !p.scatter || p.resid_out || p.r2 || p.resid || p.bic_map;
+  if (need_resid && !h->dmma_resid) {
+    launch_epilogue_ffma(h, p);
     return;
   }
-  const bool need_resid = !p.scatter || p.resid_out || p.r2 || p.resid || p.bic_map;
   const int64_t V = p.V;
   h->resid_v.ensure(sizeof(double) * V);
   h->sst_v.ensure(sizeof(double) * V);

@@ -1,0 +1,66 @@
+"""The sparse FISTA kernel (one or two voxels per warp) against the DMMA
+kernels and the oracle, at the sizes where its dispatch and its slots change.
+
+Every FP64 FISTA kernel adds the same products in the same order and shares
+the update, so coefficients, iteration counts and flags are compared bit for
+bit; the oracle comparison uses the parity bounds (coefficients 1e-5 per
+voxel, iterations within 1: a stopping decision within rounding of tol).
+"""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+KEYS = ("coef64", "coefficients", "iterations", "converged")
+
+
+def tiled(v, seed=41):
+    """A (v, 1, 1) volume that repeats 96 phantom voxels (the last one zero)."""
+    from cs_dmri_b200.phantom import make_phantom
+    ph = make_phantom((12, 8, 1), seed=seed)
+    rows = ph.data.reshape(96, -1).copy()
+    rows[95] = 0.0
+    data = rows[np.arange(v) % 96].reshape(v, 1, 1, -1)
+    return ph, data, np.ones((v, 1, 1), bool)
+
+
+def fit(ph, data, mask, **kw):
+    from cs_dmri_b200 import shore_fit
+    return shore_fit(data, ph.bvals, ph.bvecs, mask, big_delta=ph.big_delta, small_delta=ph.small_delta,
+                     return_coef64=True, diagnostics=True, **kw)
+
+
+@pytest.mark.parametrize("order", [4, 6])
+@pytest.mark.parametrize("v", [1, 33, 601, 9475, 9999])  # order 6: two voxels per warp from 9,473
+@pytest.mark.parametrize("kw", [dict(alpha_mode="fixed", alpha=0.01),
+                                dict(alpha_mode="fixed", alpha=0.02, non_negative=True, max_iter=37),
+                                dict(alpha_mode="alpha-ratio", alpha_ratio=0.01)])
+def test_matches_the_dmma_kernel_bit_for_bit(order, v, kw):
+    from cs_dmri_b200 import _abi
+    ph, data, mask = tiled(v)
+    sparse = fit(ph, data, mask, radial_order=order, **kw)
+    _abi.set_option(_abi.OPT_FISTA_SHAPE, 16)
+    try:
+        dmma = fit(ph, data, mask, radial_order=order, **kw)
+    finally:
+        _abi.set_option(_abi.OPT_FISTA_SHAPE, 0)
+    for k in KEYS:
+        np.testing.assert_array_equal(sparse[k], dmma[k])
+
+
+@pytest.mark.parametrize("v", [14209, 14304])  # two voxels per warp from 14,209
+def test_order_8_two_voxels_per_warp_equal_one(v, oracle):
+    ph, data, mask = tiled(v)
+    two = fit(ph, data, mask, radial_order=8, alpha_mode="fixed", alpha=0.01)
+    one = fit(ph, data[:96], mask[:96], radial_order=8, alpha_mode="fixed", alpha=0.01)
+    at = np.arange(v) % 96
+    np.testing.assert_array_equal(two["coef64"], one["coef64"][at])
+    np.testing.assert_array_equal(two["converged"], one["converged"][at])
+    np.testing.assert_array_equal(two["iterations"].ravel(), one["iterations"].ravel()[at])
+    ref = oracle.shore_fit(data[:96], ph.bvals, ph.bvecs, mask[:96], big_delta=ph.big_delta,
+                           small_delta=ph.small_delta, radial_order=8, alpha_mode="fixed", alpha=0.01,
+                           diagnostics=True)
+    num = np.linalg.norm(one["coef64"] - ref["coef64"], axis=1)
+    assert (num <= 1e-5 * np.linalg.norm(ref["coef64"], axis=1)).all()
+    assert np.abs(one["iterations"].astype(int) - ref["iterations"].astype(int)).max() <= 1
