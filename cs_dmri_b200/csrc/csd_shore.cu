@@ -306,6 +306,7 @@ struct csd_handle {
   DevBuf iota;
   // differentiable fit: adjoint solution w, overflow list and its count, RTOP constants
   DevBuf adjW, adjovf, adjstat, adjconst;
+  DevBuf ppark;  // voxels the DMMA path kernel leaves to the sparse one
   DevBuf gdtab, gdq;  // per-voxel-design fit: gradient table, queue and iteration count
   int adjconst_order = -1;
   double adjconst_zeta = 0.0;
@@ -728,30 +729,19 @@ void ensure_sched(csd_handle* h, int64_t V) {
   h->schedCnt.ensure(kSchedSlotBytes * kSchedSlots);
 }
 
-template <int MT, int WARPS, bool NONNEG>
-void launch_fista_v3_n(csd_handle* h, const csd::FistaParams& p) {
-  constexpr int KP = 8 * MT;
-  // Gram tiles + per-warp y and b buffers
-  const size_t smem = sizeof(double) * (2 * static_cast<size_t>(MT) * MT * 32 + WARPS * 2 * KP * 8);
-  CSD_CUDA(cudaFuncSetAttribute(csd::k_fista_v3<MT, WARPS, NONNEG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(smem)));
-  int per_sm = 0;
-  CSD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, csd::k_fista_v3<MT, WARPS, NONNEG>, 32 * WARPS, smem));
-  per_sm = std::max(per_sm, 1);
-  const int64_t warps_needed = (p.n_work + 7) / 8;
-  const int sms = h->sm_cap > 0 ? std::min(h->sm_cap, h->num_sms) : h->num_sms;
-  int64_t blocks = std::min<int64_t>(static_cast<int64_t>(sms) * per_sm, (warps_needed + WARPS - 1) / WARPS);
-  blocks = std::max<int64_t>(blocks, 1);
+// One FISTA launch, or the two-pass schedule: pass 1 to the cap, the parked
+// voxels ordered, pass 2 resuming them.  go(params) launches the kernel, whose
+// grid holds `slots` voxels at a time.
+template <class Go>
+void launch_fista_sched(csd_handle* h, const csd::FistaParams& p, int64_t slots, Go go) {
   csd::FistaParams q = p;
   q.gfrag = h->gfrag.as<double>();
   q.mom = h->mom.as<double>();
   cudaStream_t st = h->stream;
-  if (!sched_enabled(h, p, blocks * WARPS * 8)) {
-    csd::k_fista_v3<MT, WARPS, NONNEG><<<static_cast<unsigned>(blocks), 32 * WARPS, smem, st>>>(q);
-    CSD_LAUNCH();
+  if (!sched_enabled(h, p, slots)) {
+    go(q);
     return;
   }
-  // pass 1 to the cap; order the parked voxels; pass 2 resumes them
   if (h->sched_slot < 0 || h->sched_slot >= kSchedSlots || h->sched_base < 0 || h->sched_base + p.n_work > p.V)
     throw Error{CSD_ERR_INVALID, "two-pass FISTA schedule: slot or base out of range"};
   ensure_sched(h, p.V);
@@ -770,8 +760,7 @@ void launch_fista_v3_n(csd_handle* h, const csd::FistaParams& p) {
   q1.pend = pend;
   q1.pend_key = key;
   q1.n_pend = n_pend;
-  csd::k_fista_v3<MT, WARPS, NONNEG><<<static_cast<unsigned>(blocks), 32 * WARPS, smem, st>>>(q1);
-  CSD_LAUNCH();
+  go(q1);
   csd::k_sched_hist<<<h->num_sms, 256, 0, st>>>(key, n_pend, hist, p.iter_total ? p.iter_total + 2 : nullptr);
   CSD_LAUNCH();
   csd::k_sched_order<<<h->num_sms, csd::kSchedBins, 0, st>>>(pend, key, n_pend, hist, cursor, order);
@@ -784,8 +773,27 @@ void launch_fista_v3_n(csd_handle* h, const csd::FistaParams& p) {
   q2.n_work_dev = n_pend;
   q2.pend = nullptr;
   q2.pend_key = nullptr;
-  csd::k_fista_v3<MT, WARPS, NONNEG><<<static_cast<unsigned>(blocks), 32 * WARPS, smem, st>>>(q2);
-  CSD_LAUNCH();
+  go(q2);
+}
+
+template <int MT, int WARPS, bool NONNEG>
+void launch_fista_v3_n(csd_handle* h, const csd::FistaParams& p) {
+  constexpr int KP = 8 * MT;
+  // Gram tiles + per-warp y and b buffers
+  const size_t smem = sizeof(double) * (2 * static_cast<size_t>(MT) * MT * 32 + WARPS * 2 * KP * 8);
+  auto* kern = csd::k_fista_v3<MT, WARPS, NONNEG>;
+  CSD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  int per_sm = 0;
+  CSD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * WARPS, smem));
+  per_sm = std::max(per_sm, 1);
+  const int64_t warps_needed = (p.n_work + 7) / 8;
+  const int sms = h->sm_cap > 0 ? std::min(h->sm_cap, h->num_sms) : h->num_sms;
+  const int64_t blocks = std::max<int64_t>(
+      1, std::min<int64_t>(static_cast<int64_t>(sms) * per_sm, (warps_needed + WARPS - 1) / WARPS));
+  launch_fista_sched(h, p, blocks * WARPS * 8, [&](const csd::FistaParams& q) {
+    kern<<<static_cast<unsigned>(blocks), 32 * WARPS, smem, h->stream>>>(q);
+    CSD_LAUNCH();
+  });
 }
 
 template <int MT, int WARPS>
@@ -867,6 +875,113 @@ void launch_fista_sparse(csd_handle* h, const csd::FistaParams& p) {
       break;
     default: throw Error{CSD_ERR_INVALID, "the sparse FISTA kernel is built for radial orders 4, 6 and 8"};
   }
+}
+
+// The fused alpha path over p.f.n_work voxels.
+template <int K, int P, int MAXWARPS, int MINCTAS, bool NONNEG>
+void launch_path_sparse_t(csd_handle* h, const csd::PathParams& p) {
+  using S = csd::SparseShape<K, P>;
+  const int64_t need = (p.f.n_work + P - 1) / P;
+  const int warps =
+      static_cast<int>(std::min<int64_t>(MAXWARPS, std::max<int64_t>(4, (need + h->num_sms - 1) / h->num_sms)));
+  const size_t smem = S::G_BYTES + static_cast<size_t>(warps) * S::WARP_BYTES;
+  auto* kern = csd::k_path_sparse<K, P, MAXWARPS, MINCTAS, NONNEG>;
+  CSD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  const int64_t blocks = std::max<int64_t>(
+      1, std::min<int64_t>(static_cast<int64_t>(h->num_sms) * MINCTAS, (need + warps - 1) / warps));
+  csd::PathParams q = p;
+  q.f.G = h->G.as<double>();
+  q.f.mom = h->mom.as<double>();
+  kern<<<static_cast<unsigned>(blocks), 32 * warps, smem, h->stream>>>(q);
+  CSD_LAUNCH();
+}
+
+template <int K, int P, int MAXWARPS, int MINCTAS>
+void launch_path_sparse_p(csd_handle* h, const csd::PathParams& p) {
+  if (p.f.non_negative)
+    launch_path_sparse_t<K, P, MAXWARPS, MINCTAS, true>(h, p);
+  else
+    launch_path_sparse_t<K, P, MAXWARPS, MINCTAS, false>(h, p);
+}
+
+template <int MT, int WARPS, bool NONNEG>
+void launch_path_dmma_n(csd_handle* h, const csd::PathParams& p, int park_at) {
+  const size_t smem =
+      sizeof(double) * (2 * static_cast<size_t>(MT) * MT * 32 + WARPS * static_cast<size_t>(csd::kPathWarpDoubles<MT>));
+  auto* kern = csd::k_path_dmma<MT, WARPS, NONNEG>;
+  CSD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  int per_sm = 0;
+  CSD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * WARPS, smem));
+  // a short list on fewer warps per CTA, so that every SM has some
+  const int64_t groups = (p.f.n_work + 7) / 8;
+  const int warps = static_cast<int>(
+      std::min<int64_t>(WARPS, std::max<int64_t>(4, (groups + h->num_sms - 1) / h->num_sms)));
+  const int64_t blocks = std::max<int64_t>(
+      1, std::min<int64_t>(static_cast<int64_t>(h->num_sms) * std::max(per_sm, 1), (groups + warps - 1) / warps));
+  csd::PathParams q = p;
+  q.f.gfrag = h->gfrag.as<double>();
+  q.f.mom = h->mom.as<double>();
+  kern<<<static_cast<unsigned>(blocks), 32 * warps, smem, h->stream>>>(q, park_at);
+  CSD_LAUNCH();
+}
+
+template <int MT, int WARPS>
+void launch_path_dmma_p(csd_handle* h, const csd::PathParams& p, int park_at) {
+  if (p.f.non_negative)
+    launch_path_dmma_n<MT, WARPS, true>(h, p, park_at);
+  else
+    launch_path_dmma_n<MT, WARPS, false>(h, p, park_at);
+}
+
+// The fused path: from kPathDmmaVoxels voxels per SM on the DMMA slots, its
+// last voxels on the sparse kernel; below that (and at order 8) on the sparse
+// kernel alone.  Measured, DMMA / sparse (two voxels per warp) / point by
+// point: L2-anchored 4,000 voxels 18.7 / 12.9 / 18.1 ms, 30,211 voxels (N =
+// 181) 44.8 / 53.3 / 59.9 ms, 148,877 voxels 159 / 247 / 184 ms; path-BIC
+// 8,000 voxels 35.6 / 34.4 / 41.8 ms, 64,000 voxels 130 / 205 / 207 ms; order
+// 4, 64,000 voxels 22 / 36 / 40 ms.
+constexpr int kPathDmmaVoxels = 64;
+constexpr int kPathParkAt = 4;  // active slots of a warp at which it parks them: 0 47.6, 2 45.7, 4 44.8, 6 47.2 ms
+
+void launch_path_fused(csd_handle* h, const csd::PathParams& p0) {
+  csd::PathParams p = p0;
+  const int64_t V = p.f.n_work;
+  cudaStream_t st = h->stream;
+  if (h->K != 145 && V >= kPathDmmaVoxels * h->num_sms) {
+    h->schedY.ensure(sizeof(double) * static_cast<size_t>(V) * h->Kp);
+    h->schedD.ensure(sizeof(double) * static_cast<size_t>(V) * h->Kp);
+    h->ppark.ensure(16 + sizeof(csd::PathPark) * static_cast<size_t>(V));
+    p.n_park = h->ppark.as<unsigned long long>();
+    p.park = reinterpret_cast<csd::PathPark*>(static_cast<char*>(h->ppark.p) + 16);
+    p.Xp = h->schedD.as<double>();
+    p.Yp = h->schedY.as<double>();
+    CSD_CUDA(cudaMemsetAsync(p.n_park, 0, sizeof(unsigned long long), st));
+    if (h->K == 29)
+      launch_path_dmma_p<4, 16>(h, p, kPathParkAt);
+    else
+      launch_path_dmma_p<9, 16>(h, p, kPathParkAt);
+    CSD_CUDA(cudaMemsetAsync(p.f.queue, 0, sizeof(unsigned long long), st));
+    p.resume = 1;
+  }
+  switch (h->K) {
+    case 29: launch_path_sparse_p<29, 1, 16, 2>(h, p); break;
+    case 72:
+      if (!p.resume && V > 16 * h->num_sms)
+        launch_path_sparse_p<72, 2, 16, 1>(h, p);
+      else
+        launch_path_sparse_p<72, 1, 16, 2>(h, p);
+      break;
+    case 145: launch_path_sparse_p<145, 1, 16, 1>(h, p); break;
+    default: throw Error{CSD_ERR_INVALID, "the fused alpha path is built for radial orders 4, 6 and 8"};
+  }
+}
+
+// Whether a path strategy runs as the fused kernel: FP64 with the kernel shape
+// left to the library.  The mixed precision and a forced shape walk the path
+// point by point.
+bool fused_path(const csd_handle* h, const csd_shore_spec* spec) {
+  return spec->precision == CSD_PRECISION_FP64 && h->opt_shape == 0 && spec->max_iter > 0 &&
+         (h->K == 29 || h->K == 72 || h->K == 145);
 }
 
 // FISTA kernel variant: 0 = k_fista_fp64 (registers hold x, y, b); 3 / 4 =
@@ -1950,48 +2065,15 @@ FitInfo run_fit(csd_handle* h, const float* d_data, const uint8_t* d_mask, int64
       } else {
         // Path strategies (src/solver/alpha.rs:249-318).
         const int P = spec->path_n_alphas;
-        h->Xsel.ensure(sizeof(double) * V * Kp);
-        h->Xfb.ensure(sizeof(double) * V * Kp);
-        h->list.ensure(sizeof(int64_t) * V);
-        h->active.ensure(V);
-        h->pbest.ensure(sizeof(double) * V);
-        h->psel.ensure(V);
-        h->palpha_sel.ensure(sizeof(double) * V);
-        h->pit_sel.ensure(sizeof(uint32_t) * V);
-        h->pconv_sel.ensure(V);
-        h->palpha_fb.ensure(sizeof(double) * V);
-        h->pit_fb.ensure(sizeof(uint32_t) * V);
-        h->pconv_fb.ensure(V);
-        h->pcode.ensure(V);
-        CSD_CUDA(cudaMemsetAsync(h->Xsel.p, 0, sizeof(double) * V * Kp, st));
-        CSD_CUDA(cudaMemsetAsync(h->psel.p, 0, V, st));
-        CSD_CUDA(cudaMemsetAsync(h->palpha_sel.p, 0, sizeof(double) * V, st));
-        CSD_CUDA(cudaMemsetAsync(h->pit_sel.p, 0, sizeof(uint32_t) * V, st));
-        CSD_CUDA(cudaMemsetAsync(h->pconv_sel.p, 1, V, st));
-        {
-          // best metric starts at +inf
-          csd::k_fill_f64<<<grid1(V), 256, 0, st>>>(h->pbest.as<double>(), V, INFINITY);
-          CSD_LAUNCH();
-        }
-        csd::PathState ps{};
-        ps.best = h->pbest.as<double>();
-        ps.selected = h->psel.as<uint8_t>();
-        ps.active = h->active.as<uint8_t>();
-        ps.alpha_sel = h->palpha_sel.as<double>();
-        ps.it_sel = h->pit_sel.as<uint32_t>();
-        ps.conv_sel = h->pconv_sel.as<uint8_t>();
-        ps.alpha_fb = h->palpha_fb.as<double>();
-        ps.it_fb = h->pit_fb.as<uint32_t>();
-        ps.conv_fb = h->pconv_fb.as<uint8_t>();
-        ps.copy_code = h->pcode.as<int8_t>();
-        csd::k_init_active<<<grid1(V), 256, 0, st>>>(V, h->zero.as<uint8_t>(), h->active.as<uint8_t>());
-        CSD_LAUNCH();
         const double* rss_l2 = nullptr;
         if (mode == CSD_ALPHA_L2_ANCHORED) {
           // Tikhonov reference RSS per voxel (src/fit.rs:436-438).
           h->Xl2.ensure(sizeof(double) * V * Kp);
           h->rss_l2.ensure(sizeof(double) * V);
-          launch_tikhonov(h, h->B.as<double>(), h->Xl2.as<double>(), V);
+          if (h->dmma_rhs && h->pfrag_valid && !data_on_host)  // one product, as the L2 fit
+            launch_rhs(h, d_data, V, nullptr, h->pfrag.as<double>(), h->Xl2.as<double>());
+          else
+            launch_tikhonov(h, h->B.as<double>(), h->Xl2.as<double>(), V);
           csd::EpilogueParams rp = ep;
           rp.X = h->Xl2.as<double>();
           rp.scatter = false;
@@ -2001,51 +2083,109 @@ FitInfo run_fit(csd_handle* h, const float* d_data, const uint8_t* d_mask, int64
           CSD_LAUNCH();
           rss_l2 = h->rss_l2.as<double>();
         }
-        record(h, 6);
-        int64_t n_work = 0;
-        for (int i = 0; i < P; ++i) {
-          n_work = compact(h, h->active.as<uint8_t>(), V, h->list);
-          if (n_work == 0) break;
-          csd::k_path_alpha<<<grid1(n_work), 256, 0, st>>>(h->amax.as<double>(), h->list.as<int64_t>(),
-                                                           n_work, i, P, path_eps, h->alpha_v.as<double>());
-          CSD_LAUNCH();
-          fp.alpha_v = h->alpha_v.as<double>();
-          fp.warm = (i == 0) ? nullptr : h->X.as<double>();
-          fp.list = h->list.as<int64_t>();
-          fp.n_work = n_work;
+        if (fused_path(h, spec)) {
+          csd::PathParams pp{};
+          pp.f = fp;
+          pp.amax = h->amax.as<double>();
+          pp.rss_l2 = rss_l2;
+          pp.alpha = h->alpha_v.as<double>();
+          pp.data = d_data;
+          pp.vox = h->vox.as<int64_t>();
+          pp.sig = h->sig_compact;
+          pp.Mt = h->Mt.as<double>();
+          pp.N = N;
+          pp.n_alphas = P;
+          pp.mode = mode;
+          pp.eps = path_eps;
+          pp.slack = spec->slack;
           CSD_CUDA(cudaMemsetAsync(h->queue.p, 0, sizeof(unsigned long long), st));
-          launch_fista(h, MT, fp);
-          csd::EpilogueParams rp = ep;
-          rp.X = h->X.as<double>();
-          rp.scatter = false;
-          rp.resid_out = h->resid_v.as<double>();
-          rp.nnz_out = h->nnz_v.as<int>();
-          rp.list = h->list.as<int64_t>();
-          rp.n_work = n_work;
-          launch_epilogue(h, rp);
-          csd::k_path_update<<<grid1(n_work), 256, 0, st>>>(
-              mode, h->list.as<int64_t>(), n_work, N, h->resid_v.as<double>(), h->nnz_v.as<int>(),
-              h->alpha_v.as<double>(), h->iters.as<uint32_t>(), h->conv.as<uint8_t>(), rss_l2,
-              spec->slack, ps);
+          record(h, 6);
+          launch_path_fused(h, pp);
+          record(h, 7);
+          alpha_final = h->alpha_v.as<double>();
+        } else {
+          h->Xsel.ensure(sizeof(double) * V * Kp);
+          h->Xfb.ensure(sizeof(double) * V * Kp);
+          h->list.ensure(sizeof(int64_t) * V);
+          h->active.ensure(V);
+          h->pbest.ensure(sizeof(double) * V);
+          h->psel.ensure(V);
+          h->palpha_sel.ensure(sizeof(double) * V);
+          h->pit_sel.ensure(sizeof(uint32_t) * V);
+          h->pconv_sel.ensure(V);
+          h->palpha_fb.ensure(sizeof(double) * V);
+          h->pit_fb.ensure(sizeof(uint32_t) * V);
+          h->pconv_fb.ensure(V);
+          h->pcode.ensure(V);
+          CSD_CUDA(cudaMemsetAsync(h->Xsel.p, 0, sizeof(double) * V * Kp, st));
+          CSD_CUDA(cudaMemsetAsync(h->psel.p, 0, V, st));
+          CSD_CUDA(cudaMemsetAsync(h->palpha_sel.p, 0, sizeof(double) * V, st));
+          CSD_CUDA(cudaMemsetAsync(h->pit_sel.p, 0, sizeof(uint32_t) * V, st));
+          CSD_CUDA(cudaMemsetAsync(h->pconv_sel.p, 1, V, st));
+          {
+            // best metric starts at +inf
+            csd::k_fill_f64<<<grid1(V), 256, 0, st>>>(h->pbest.as<double>(), V, INFINITY);
+            CSD_LAUNCH();
+          }
+          csd::PathState ps{};
+          ps.best = h->pbest.as<double>();
+          ps.selected = h->psel.as<uint8_t>();
+          ps.active = h->active.as<uint8_t>();
+          ps.alpha_sel = h->palpha_sel.as<double>();
+          ps.it_sel = h->pit_sel.as<uint32_t>();
+          ps.conv_sel = h->pconv_sel.as<uint8_t>();
+          ps.alpha_fb = h->palpha_fb.as<double>();
+          ps.it_fb = h->pit_fb.as<uint32_t>();
+          ps.conv_fb = h->pconv_fb.as<uint8_t>();
+          ps.copy_code = h->pcode.as<int8_t>();
+          csd::k_init_active<<<grid1(V), 256, 0, st>>>(V, h->zero.as<uint8_t>(), h->active.as<uint8_t>());
           CSD_LAUNCH();
-          csd::k_path_copy<<<grid1(n_work * Kp), 256, 0, st>>>(h->list.as<int64_t>(), n_work, Kp,
-                                                               h->pcode.as<int8_t>(), h->X.as<double>(),
-                                                               h->Xsel.as<double>(), h->Xfb.as<double>());
+          record(h, 6);
+          int64_t n_work = 0;
+          for (int i = 0; i < P; ++i) {
+            n_work = compact(h, h->active.as<uint8_t>(), V, h->list);
+            if (n_work == 0) break;
+            csd::k_path_alpha<<<grid1(n_work), 256, 0, st>>>(h->amax.as<double>(), h->list.as<int64_t>(),
+                                                             n_work, i, P, path_eps, h->alpha_v.as<double>());
+            CSD_LAUNCH();
+            fp.alpha_v = h->alpha_v.as<double>();
+            fp.warm = (i == 0) ? nullptr : h->X.as<double>();
+            fp.list = h->list.as<int64_t>();
+            fp.n_work = n_work;
+            CSD_CUDA(cudaMemsetAsync(h->queue.p, 0, sizeof(unsigned long long), st));
+            launch_fista(h, MT, fp);
+            csd::EpilogueParams rp = ep;
+            rp.X = h->X.as<double>();
+            rp.scatter = false;
+            rp.resid_out = h->resid_v.as<double>();
+            rp.nnz_out = h->nnz_v.as<int>();
+            rp.list = h->list.as<int64_t>();
+            rp.n_work = n_work;
+            launch_epilogue(h, rp);
+            csd::k_path_update<<<grid1(n_work), 256, 0, st>>>(
+                mode, h->list.as<int64_t>(), n_work, N, h->resid_v.as<double>(), h->nnz_v.as<int>(),
+                h->alpha_v.as<double>(), h->iters.as<uint32_t>(), h->conv.as<uint8_t>(), rss_l2,
+                spec->slack, ps);
+            CSD_LAUNCH();
+            csd::k_path_copy<<<grid1(n_work * Kp), 256, 0, st>>>(h->list.as<int64_t>(), n_work, Kp,
+                                                                 h->pcode.as<int8_t>(), h->X.as<double>(),
+                                                                 h->Xsel.as<double>(), h->Xfb.as<double>());
+            CSD_LAUNCH();
+          }
+          if (mode == CSD_ALPHA_L2_ANCHORED) {
+            csd::k_path_finalize<<<grid1(V * Kp), 256, 0, st>>>(V, Kp, h->zero.as<uint8_t>(), ps,
+                                                                 h->Xfb.as<double>(), h->Xsel.as<double>());
+            CSD_LAUNCH();
+          }
+          record(h, 7);
+          Xfinal = h->Xsel.as<double>();
+          it_final = h->pit_sel.as<uint32_t>();
+          conv_final = h->pconv_sel.as<uint8_t>();
+          alpha_final = h->palpha_sel.as<double>();
+          csd::k_zero_voxels<<<grid1(V), 256, 0, st>>>(V, h->zero.as<uint8_t>(), h->palpha_sel.as<double>(),
+                                                       h->pit_sel.as<uint32_t>(), h->pconv_sel.as<uint8_t>());
           CSD_LAUNCH();
         }
-        if (mode == CSD_ALPHA_L2_ANCHORED) {
-          csd::k_path_finalize<<<grid1(V * Kp), 256, 0, st>>>(V, Kp, h->zero.as<uint8_t>(), ps,
-                                                               h->Xfb.as<double>(), h->Xsel.as<double>());
-          CSD_LAUNCH();
-        }
-        record(h, 7);
-        Xfinal = h->Xsel.as<double>();
-        it_final = h->pit_sel.as<uint32_t>();
-        conv_final = h->pconv_sel.as<uint8_t>();
-        alpha_final = h->palpha_sel.as<double>();
-        csd::k_zero_voxels<<<grid1(V), 256, 0, st>>>(V, h->zero.as<uint8_t>(), h->palpha_sel.as<double>(),
-                                                     h->pit_sel.as<uint32_t>(), h->pconv_sel.as<uint8_t>());
-        CSD_LAUNCH();
       }
     }
   }
@@ -2594,7 +2734,7 @@ void csd_destroy(csd_handle* h) {
                     &h->iota, &h->adjW, &h->adjovf, &h->adjstat, &h->adjconst, &h->hinv,
                     &h->gdtab, &h->gdq, &h->tuneB, &h->tuneX, &h->tuneIt, &h->tuneConv, &h->tuneQ,
                     &h->schedY, &h->schedPend, &h->schedKey, &h->schedOrder, &h->schedCnt,
-                    &h->schedD, &h->schedU, &h->schedN, &h->gtf32, &h->x32, &h->kktv, &h->kktovf,
+                    &h->schedD, &h->schedU, &h->schedN, &h->ppark, &h->gtf32, &h->x32, &h->kktv, &h->kktovf,
                     &h->kktfail, &h->kktstat};
   for (auto s : h->pipe)
     if (s) cudaStreamSynchronize(s);

@@ -400,6 +400,89 @@ __global__ void __launch_bounds__(256) k_fista_fp64(FistaParams p) {
   }
 }
 
+// The key of a voxel parked at iteration `cap`: the iterations it still needs
+// over 2^16, from the least-squares line through log2(rel^2) over iterations
+// w0 + 1 .. cap (sl, skl: its sums of log2(rel^2) and k log2(rel^2)) extended
+// to log2(tol^2); no decrease: the most.
+__device__ __forceinline__ float park_key(float sl, float skl, int cap, int w0, double tol) {
+  const float n = static_cast<float>(cap - w0), km = 0.5f * (n + 1.f);
+  const float lm = sl / n;
+  const float sxx = n * (n * n - 1.f) / 12.f;
+  const float slope = (skl - km * sl) / sxx;
+  const float lc = lm + slope * (n - km);
+  const float target = 2.f * log2f(static_cast<float>(tol));
+  const float rem = slope < 0.f ? (target - lc) / slope : 65536.f;
+  return fminf(fmaxf(rem, 1.f), 65536.f) * (1.f / 65536.f);
+}
+
+// One iteration of a warp's eight voxel slots: G y over the k-steps marked in
+// `live` (words of 32; a superset of those with a non-zero y entry), the update
+// of x and of y in ybuf ([k][voxel]; b thread-private in bbuf, [mt][lane][2]),
+// the marks of the new y, and per voxel the sums of d^2 and x^2 over its rows
+// (src/solver/fista.rs:89-113).  Returns the k-steps executed.
+template <int MT, bool NONNEG>
+__device__ __forceinline__ unsigned dmma_fista_step(const double* sG, double* ybuf, const double* bbuf,
+                                                    unsigned (&live)[(2 * MT + 31) / 32], double (&x)[MT][2],
+                                                    const double (&mom)[2], const double (&thr)[2], double c, int lane,
+                                                    double (&dx2)[2], double (&xn2)[2]) {
+  constexpr int KT = 2 * MT, LW = (KT + 31) / 32;
+  const int g = lane >> 2, q = lane & 3;
+  unsigned ksteps = 0;
+  double acc[MT][2];
+#pragma unroll
+  for (int mt = 0; mt < MT; ++mt) acc[mt][0] = acc[mt][1] = 0.0;
+  // A k-step whose four y entries are exactly zero for all eight voxels adds
+  // only zeros (soft thresholding keeps most of y at 0): only the live ones run.
+#pragma unroll
+  for (int w = 0; w < LW; ++w) {
+    unsigned m = live[w] & (KT - 32 * w >= 32 ? kFull : (1u << (KT - 32 * w)) - 1u);
+    ksteps += __popc(m);
+#pragma unroll 1
+    for (; m != 0; m &= m - 1) {
+      const int kt = 32 * w + __ffs(static_cast<int>(m)) - 1;
+      const double bf = ybuf[(4 * kt + q) * 8 + g];
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt) dmma_m8n8k4(acc[mt][0], acc[mt][1], sG[(mt * KT + kt) * 32 + lane], bf);
+    }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < 2; ++j) dx2[j] = xn2[j] = 0.0;
+#pragma unroll
+  for (int w = 0; w < LW; ++w) live[w] = 0u;
+#pragma unroll
+  for (int mt = 0; mt < MT; ++mt) {
+    const int row = 8 * mt + g;
+    const double2 yv = *reinterpret_cast<const double2*>(&ybuf[row * 8 + 2 * q]);
+    const double2 bv = *reinterpret_cast<const double2*>(&bbuf[(mt * 32 + lane) * 2]);
+    const double yy[2] = {yv.x, yv.y}, bb[2] = {bv.x, bv.y};
+    double yo[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const double xn = fista_prox<NONNEG>(acc[mt][j], bb[j], yy[j], c, thr[j]);
+      const double d = __dsub_rn(xn, x[mt][j]);
+      yo[j] = fma(mom[j], d, xn);
+      dx2[j] = fma(d, d, dx2[j]);
+      xn2[j] = fma(xn, xn, xn2[j]);
+      x[mt][j] = xn;
+    }
+    *reinterpret_cast<double2*>(&ybuf[row * 8 + 2 * q]) = make_double2(yo[0], yo[1]);
+    if ((__double_as_longlong(yo[0]) | __double_as_longlong(yo[1])) != 0) live[mt / 16] |= 1u << (2 * (mt % 16));
+  }
+  // rows 8 mt .. 8 mt + 3 (lanes 0-15) are k-step 2 mt, the others 2 mt + 1
+#pragma unroll
+  for (int w = 0; w < LW; ++w) live[w] = __reduce_or_sync(kFull, live[w] << (g >> 2));
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) {
+      dx2[j] += __shfl_xor_sync(kFull, dx2[j], o);
+      xn2[j] += __shfl_xor_sync(kFull, xn2[j], o);
+    }
+  }
+  return ksteps;
+}
+
 // FISTA, one warp per 8 voxel slots (as k_fista_fp64) with a lighter
 // per-iteration path:
 //  * y lives only in the warp's shared B-operand buffer and b in a
@@ -511,64 +594,10 @@ __global__ void __launch_bounds__(32 * WARPS) k_fista_v3(FistaParams p) {
     executed += (g == 0) ? ((vid[0] >= 0) + (vid[1] >= 0)) : 0;
     __syncwarp();
 
-    // ---- acc = G y on the FP64 tensor cores
-    double acc[MT][2];
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt) acc[mt][0] = acc[mt][1] = 0.0;
-    // A k-step whose four y entries are exactly zero for all eight voxels adds
-    // only zeros (soft thresholding keeps most of y at 0): only the live ones run.
-#pragma unroll
-    for (int w = 0; w < LW; ++w) {
-      unsigned m = live[w] & (KT - 32 * w >= 32 ? kFull : (1u << (KT - 32 * w)) - 1u);
-      ksteps += __popc(m);
-#pragma unroll 1
-      for (; m != 0; m &= m - 1) {
-        const int kt = 32 * w + __ffs(static_cast<int>(m)) - 1;
-        const double bf = ybuf[(4 * kt + q) * 8 + g];
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt) {
-          dmma_m8n8k4(acc[mt][0], acc[mt][1], sG[(mt * KT + kt) * 32 + lane], bf);
-        }
-      }
-    }
-    __syncwarp();
-
-    // ---- proximal gradient step and momentum (fista.rs:95-113)
-    double mom[2], dx2[2] = {0.0, 0.0}, xn2[2] = {0.0, 0.0};
+    double mom[2], dx2[2], xn2[2];
 #pragma unroll
     for (int j = 0; j < 2; ++j) mom[j] = (vid[j] >= 0) ? p.mom[it[j]] : 0.0;
-#pragma unroll
-    for (int w = 0; w < LW; ++w) live[w] = 0u;
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt) {
-      const int row = 8 * mt + g;
-      const double2 yv = *reinterpret_cast<const double2*>(&ybuf[row * 8 + 2 * q]);
-      const double2 bv = *reinterpret_cast<const double2*>(&bbuf[(mt * 32 + lane) * 2]);
-      const double yy[2] = {yv.x, yv.y}, bb[2] = {bv.x, bv.y};
-      double yo[2];
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const double xn = fista_prox<NONNEG>(acc[mt][j], bb[j], yy[j], c, thr[j]);
-        const double d = __dsub_rn(xn, x[mt][j]);
-        yo[j] = fma(mom[j], d, xn);
-        dx2[j] = fma(d, d, dx2[j]);
-        xn2[j] = fma(xn, xn, xn2[j]);
-        x[mt][j] = xn;
-      }
-      *reinterpret_cast<double2*>(&ybuf[row * 8 + 2 * q]) = make_double2(yo[0], yo[1]);
-      if ((__double_as_longlong(yo[0]) | __double_as_longlong(yo[1])) != 0) live[mt / 16] |= 1u << (2 * (mt % 16));
-    }
-    // rows 8 mt .. 8 mt + 3 (lanes 0-15) are k-step 2 mt, the others 2 mt + 1
-#pragma unroll
-    for (int w = 0; w < LW; ++w) live[w] = __reduce_or_sync(kFull, live[w] << (g >> 2));
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-#pragma unroll
-      for (int o = 4; o < 32; o <<= 1) {
-        dx2[j] += __shfl_xor_sync(kFull, dx2[j], o);
-        xn2[j] += __shfl_xor_sync(kFull, xn2[j], o);
-      }
-    }
+    ksteps += dmma_fista_step<MT, NONNEG>(sG, ybuf, bbuf, live, x, mom, thr, c, lane, dx2, xn2);
 
     // ---- per-voxel stopping rule (fista.rs:115-127) and write-out
 #pragma unroll
@@ -609,16 +638,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_fista_v3(FistaParams p) {
         if (g == 0) {
           const unsigned long long slot = atomicAdd(p.n_pend, 1ull);
           p.pend[slot] = v;
-          // remaining iterations: the least-squares line through log2(rel^2)
-          // over the window, extended to log2(tol^2) (no decrease: the most)
-          const float n = static_cast<float>(p.cap - w0), km = 0.5f * (n + 1.f);
-          const float lm = sl[j] / n;
-          const float sxx = n * (n * n - 1.f) / 12.f;
-          const float slope = (skl[j] - km * sl[j]) / sxx;
-          const float lc = lm + slope * (n - km);
-          const float target = 2.f * log2f(static_cast<float>(p.tol));
-          const float rem = slope < 0.f ? (target - lc) / slope : 65536.f;
-          p.pend_key[slot] = fminf(fmaxf(rem, 1.f), 65536.f) * (1.f / 65536.f);
+          p.pend_key[slot] = park_key(sl[j], skl[j], p.cap, w0, p.tol);
         }
         need[j] = true;
         vid[j] = -1;

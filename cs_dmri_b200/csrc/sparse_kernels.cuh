@@ -342,4 +342,447 @@ __global__ void __launch_bounds__(32 * MAXWARPS, MINCTAS) k_fista_sparse(FistaPa
   if (p.iter_total && f.lane == 0 && executed) atomicAdd(p.iter_total, executed);
 }
 
+// ------------------------------------------------------- alpha path, fused
+
+// A voxel in mid-path: where it stands, its x and y in rows v of Xp and Yp.
+struct PathPark {
+  double best;
+  int v, point, it, pad;
+};
+
+struct PathParams {
+  FistaParams f;         // B, X (the chosen point's coefficients), iters, conv, step, n_inv, tol, max_iter, queue
+  const double* amax;    // V: alpha_max
+  const double* rss_l2;  // V: the Tikhonov fit's RSS (PathL2Anchored), or nullptr
+  double* alpha;         // V out
+  const float* data;     // signals: row vox[v] of `data`, or row v of `sig`
+  const int64_t* vox;
+  const float* sig;
+  const double* Mt;      // KP x N, transposed design
+  int N, n_alphas, mode; // mode 2 = PathBic, 3 = PathL2Anchored
+  double eps, slack;
+  // k_path_dmma leaves the voxels of its last warps here for k_path_sparse
+  PathPark* park;
+  unsigned long long* n_park;
+  double *Xp, *Yp;       // V x KP
+  int resume;            // take the parked voxels (*n_park of them) instead of 0 .. n_work-1
+};
+
+// Point i of log_path(alpha_max, n, eps) (src/solver/alpha.rs:57-69).
+__device__ __forceinline__ double path_alpha(double amax, int i, int n, double eps) {
+  const double lmax = log(amax), lmin = log(amax * eps);
+  const double t = static_cast<double>(i) / static_cast<double>(n - 1);
+  return exp(lmax + t * (lmin - lmax));
+}
+
+// Selection at one path point: PathBic keeps the lowest BIC (bic_argmin,
+// alpha.rs:107-128), PathL2Anchored the lowest RSS until one is within the
+// slack of the Tikhonov fit's, which ends the path (l2_anchored_argmax,
+// alpha.rs:140-165).
+__device__ __forceinline__ bool path_better(int mode, int N, int nnz, double rss, double rss_limit, double& best,
+                                            bool& last) {
+  if (mode == 2) {
+    const double n = static_cast<double>(N);
+    const double bic = n * log(fmax(rss, 2.2250738585072014e-308) / n) + log(n) * static_cast<double>(nnz);
+    if (!(bic < best)) return false;
+    best = bic;
+    return true;
+  }
+  const bool within = rss <= rss_limit;
+  last = last || within;
+  if (!within && !(rss < best)) return false;
+  best = rss;
+  return true;
+}
+
+// ||s - M c||^2 of one voxel on a warp, c sparse (listed in increasing row as
+// values, every P-th double, and rows): four samples a lane and
+// four coefficients at a time, so 16 loads are in flight; the columns of M are
+// read from M^T (coalesced, L1 / L2).
+template <int P>
+__device__ __forceinline__ double sparse_rss(const float* __restrict__ sig, const double* __restrict__ Mt, int N,
+                                             const double* val, const int* row, int nnz, int lane) {
+  double rss = 0.0;
+  for (int n0 = lane; n0 < N; n0 += 128) {
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    int off[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) off[u] = n0 + 32 * u < N ? n0 + 32 * u : N - 1;
+#pragma unroll 4
+    for (int e = 0; e < nnz; ++e) {
+      const double c = val[P * e];
+      const double* col = Mt + static_cast<size_t>(row[e]) * N;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) acc[u] = fma(__ldg(col + off[u]), c, acc[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (n0 + 32 * u < N) {
+        const double r = static_cast<double>(__ldg(sig + n0 + 32 * u)) - acc[u];
+        rss = fma(r, r, rss);
+      }
+  }
+  for (int o = 16; o > 0; o >>= 1) rss += __shfl_xor_sync(kFull, rss, o);
+  return rss;
+}
+
+// The whole alpha path of a voxel on its slot (src/solver/alpha.rs:249-318):
+// FISTA at each alpha from the previous point's answer, the residual and the
+// selection between them, no pass over the volume per alpha.  A point's
+// coefficients are written to X when they are the best so far (PathBic: lower
+// BIC; PathL2Anchored: lower RSS, or the first within the slack, which ends the
+// path); alpha_max == 0 gives the zero result.
+//
+// Point by point over the volume (one FISTA launch, residual pass, selection
+// and compaction with a host round trip per alpha) every alpha waits for its
+// slowest voxel: 15 tails a fit.  Here a voxel's slot goes on to its next
+// alpha alone and the fit has one tail.
+template <int K, int P, int MAXWARPS, int MINCTAS, bool NONNEG>
+__global__ void __launch_bounds__(32 * MAXWARPS, MINCTAS) k_path_sparse(PathParams q) {
+  using S = SparseShape<K, P>;
+  extern __shared__ __align__(16) unsigned char sp_smem[];
+  const FistaParams& p = q.f;
+  SparseFista<K, P, NONNEG> f;
+  f.init(p.G, sp_smem);
+  __syncthreads();
+  const double c = p.step * p.n_inv;
+  unsigned long long executed = 0;
+  int64_t vid[P];
+  bool need[P];
+  int point[P];
+  double best[P], alpha[P];
+#pragma unroll
+  for (int s = 0; s < P; ++s) {
+    vid[s] = -1;
+    need[s] = true;
+    point[s] = 0;
+    best[s] = alpha[s] = 0.0;
+  }
+  const unsigned long long n_work = q.resume ? *q.n_park : static_cast<unsigned long long>(p.n_work);
+  auto set_alpha = [&](int s, int it) {
+    alpha[s] = path_alpha(q.amax[vid[s]], point[s], q.n_alphas, q.eps);
+    f.thr[s] = __dmul_rn(p.step, alpha[s]);
+    f.it[s] = it;
+    f.start(s);
+  };
+  auto store = [&](int s, int it, bool conv, double a) {
+    const int64_t v = vid[s];
+#pragma unroll
+    for (int i = 0; i < S::NR; ++i) {
+      const int row = S::row(i, f.lane);
+      if (row < S::KP) p.X[v * S::KP + row] = f.x[s][i];
+    }
+    if (f.lane == 0) {
+      p.iters[v] = static_cast<uint32_t>(it);
+      p.conv[v] = conv ? 1 : 0;
+      q.alpha[v] = a;
+    }
+  };
+  while (true) {
+#pragma unroll
+    for (int s = 0; s < P; ++s) {
+      while (need[s]) {
+        unsigned long long w = 0;
+        if (f.lane == 0) w = atomicAdd(p.queue, 1ull);
+        w = __shfl_sync(kFull, w, 0);
+        f.clear(s);
+        if (w >= n_work) {
+          vid[s] = -1;
+          need[s] = false;
+          break;
+        }
+        if (q.resume) {
+          const PathPark k = q.park[w];
+          vid[s] = k.v;
+          point[s] = k.point;
+          best[s] = k.best;
+          need[s] = false;
+#pragma unroll
+          for (int i = 0; i < S::NR; ++i) {
+            const int row = S::row(i, f.lane);
+            const bool in = row < K;
+            f.b[s][i] = in ? p.B[vid[s] * S::KP + row] : 0.0;
+            f.x[s][i] = in ? q.Xp[vid[s] * S::KP + row] : 0.0;
+            f.y[s][i] = in ? q.Yp[vid[s] * S::KP + row] : 0.0;
+          }
+          set_alpha(s, k.it);
+          break;
+        }
+        vid[s] = static_cast<int64_t>(w);
+        store(s, 0, true, 0.0);  // the zero result: kept when alpha_max == 0 or no point is ever better
+        if (q.amax[vid[s]] == 0.0) continue;
+        need[s] = false;
+#pragma unroll
+        for (int i = 0; i < S::NR; ++i) {
+          const int row = S::row(i, f.lane);
+          f.b[s][i] = row < K ? p.B[vid[s] * S::KP + row] : 0.0;
+        }
+        point[s] = 0;
+        best[s] = INFINITY;
+        set_alpha(s, 0);
+      }
+    }
+    bool any = false;
+#pragma unroll
+    for (int s = 0; s < P; ++s) any = any || vid[s] >= 0;
+    if (!any) break;
+    double mom[P];
+#pragma unroll
+    for (int s = 0; s < P; ++s) mom[s] = vid[s] >= 0 ? __ldg(p.mom + f.it[s]) : 0.0;
+    double acc[P][S::NR];
+    f.product(acc);
+#pragma unroll
+    for (int s = 0; s < P; ++s) {
+      if (vid[s] < 0) continue;
+      const bool conv = f.update(s, acc[s], mom[s], c, p.tol);
+      const int it = ++f.it[s];
+      if (!conv && it < p.max_iter) continue;
+      executed += static_cast<unsigned long long>(it);
+      // residual of this point: list its non-zero coefficients
+      const int64_t v = vid[s];
+      const unsigned lt = (1u << f.lane) - 1u;
+      int nnz = 0;
+      auto put = [&](int i, int row, bool e, int pos) {
+        sp_st_f64(f.lv + 8u * P * pos, f.x[s][i], e);
+        sp_st_s32(f.li + 4u * pos, row, e);
+      };
+#pragma unroll
+      for (int i = 0; i < S::PAIRS; ++i) {
+        const bool e = f.x[s][2 * i] != 0.0, o = f.x[s][2 * i + 1] != 0.0;
+        const unsigned me = __ballot_sync(kFull, e), mo = __ballot_sync(kFull, o);
+        const int pos = nnz + __popc(me & lt) + __popc(mo & lt);
+        put(2 * i, 64 * i + 2 * f.lane, e, pos);
+        put(2 * i + 1, 64 * i + 2 * f.lane + 1, o, pos + (e ? 1 : 0));
+        nnz += __popc(me) + __popc(mo);
+      }
+      {
+        const bool e = f.x[s][S::NR - 1] != 0.0;
+        const unsigned me = __ballot_sync(kFull, e);
+        put(S::NR - 1, 64 * S::PAIRS + f.lane, e, nnz + __popc(me & lt));
+        nnz += __popc(me);
+      }
+      __syncwarp();
+      const float* sig = q.sig ? q.sig + v * q.N : q.data + q.vox[v] * q.N;
+      const double resid = sqrt(sparse_rss<P>(sig, q.Mt, q.N, static_cast<const double*>(__cvta_shared_to_generic(f.lv)),
+                                            static_cast<const int*>(__cvta_shared_to_generic(f.li)), nnz, f.lane));
+      __syncwarp();
+      const double rss = resid * resid;
+      bool last = point[s] + 1 >= q.n_alphas;
+      const double limit = q.mode == 3 ? (1.0 + q.slack) * q.rss_l2[v] : 0.0;
+      if (path_better(q.mode, q.N, nnz, rss, limit, best[s], last)) store(s, it, conv, alpha[s]);
+      if (last) {
+        need[s] = true;
+        continue;
+      }
+      ++point[s];
+#pragma unroll
+      for (int i = 0; i < S::NR; ++i) f.y[s][i] = f.x[s][i];
+      set_alpha(s, 0);
+    }
+  }
+  if (p.iter_total && f.lane == 0 && executed) atomicAdd(p.iter_total, executed);
+}
+
+// The fused path on the DMMA slots of k_fista_v3: eight voxels to a warp, each
+// slot on its own alpha.  Along a path the iterates fill up - a voxel spends
+// most of its ~2,300 iterations at the last five of the 14 points it visits,
+// with 30-60 % of y non-zero - so the product is a dense one there and the
+// tensor cores carry it (118 SM cycles a voxel-iteration dense, against ~250
+// of k_path_sparse).  A warp whose queue is empty and whose active slots are
+// down to `park_at` leaves them to k_path_sparse, where an iteration takes a
+// third of the time: the slowest voxels would otherwise finish alone.
+template <int MT>
+constexpr int kPathWarpDoubles = 2 * (8 * MT) * 8 + (8 * MT) + (8 * MT) / 2 + 8 + 8 + 4;
+
+template <int MT, int WARPS, bool NONNEG>
+__global__ void __launch_bounds__(32 * WARPS) k_path_dmma(PathParams pp, int park_at) {
+  constexpr int KP = 8 * MT, KT = 2 * MT;
+  static_assert(KT <= 32, "one word of live k-steps");
+  extern __shared__ __align__(16) double smem_pd[];
+  const FistaParams& p = pp.f;
+  const double* sG = smem_pd;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double* ybuf = smem_pd + MT * KT * 32 + warp * kPathWarpDoubles<MT>;  // KP x 8 [k][voxel]
+  double* bbuf = ybuf + KP * 8;                                           // thread-private [mt][lane][2]
+  double* lval = bbuf + KP * 8;                                           // a point's coefficients: values ...
+  int* lrow = reinterpret_cast<int*>(lval + KP);                          // ... and rows
+  double* s_best = lval + KP + KP / 2;                                    // per slot
+  double* s_alpha = s_best + 8;
+  int* s_point = reinterpret_cast<int*>(s_alpha + 8);
+  for (int i = threadIdx.x; i < MT * KT * 32; i += blockDim.x) smem_pd[i] = p.gfrag[i];
+  __syncthreads();
+
+  const int g = lane >> 2, q = lane & 3;
+  const double tol2x4 = 4.0 * p.tol * p.tol;
+  const double c = p.step * p.n_inv;
+  const unsigned long long n_work = static_cast<unsigned long long>(p.n_work);
+  double x[MT][2];
+  int64_t vid[2] = {-1, -1};
+  int it[2] = {0, 0};
+  double thr[2] = {INFINITY, INFINITY};
+  bool need[2] = {true, true};
+  bool exhausted = false;
+  unsigned executed = 0;
+  unsigned live[1] = {kFull};
+  auto columns = [&](bool f0, bool f1) {  // the slots whose lanes set a flag
+    const unsigned n0 = __ballot_sync(kFull, lane < 4 && f0), n1 = __ballot_sync(kFull, lane < 4 && f1);
+    unsigned cols = 0;
+#pragma unroll
+    for (int l = 0; l < 4; ++l) cols |= (((n0 >> l) & 1u) << (2 * l)) | (((n1 >> l) & 1u) << (2 * l + 1));
+    return cols;
+  };
+
+  while (true) {
+    // ---- refill; a voxel with alpha_max == 0 has its zero result and its slot is filled again
+    bool refilled = false;
+    while (__any_sync(kFull, need[0] || need[1])) {
+      refilled = true;
+      const unsigned cols = columns(need[0], need[1]);
+      unsigned long long base = n_work;
+      if (!exhausted) {
+        if (lane == 0) base = atomicAdd(p.queue, static_cast<unsigned long long>(__popc(cols)));
+        base = __shfl_sync(kFull, base, 0);
+        if (base + __popc(cols) >= n_work) exhausted = true;
+      }
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        if (!need[j]) continue;
+        const int col = 2 * q + j;
+        const unsigned long long cand = base + __popc(cols & ((1u << col) - 1u));
+        const bool some = cand < n_work;
+        const int64_t v = static_cast<int64_t>(cand);
+        const double am = some ? pp.amax[v] : 0.0;
+        const bool run = some && am != 0.0;
+        need[j] = some && !run;
+        vid[j] = run ? v : -1;
+        it[j] = 0;
+        const double a = run ? path_alpha(am, 0, pp.n_alphas, pp.eps) : 0.0;
+        thr[j] = run ? __dmul_rn(p.step, a) : INFINITY;
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+          const int row = 8 * mt + g;
+          x[mt][j] = 0.0;
+          bbuf[(mt * 32 + lane) * 2 + j] = run ? p.B[v * KP + row] : 0.0;
+          ybuf[row * 8 + col] = 0.0;
+          if (some) p.X[v * KP + row] = 0.0;  // kept when alpha_max == 0 or no point is ever better
+        }
+        if (g == 0) {
+          s_best[col] = INFINITY;
+          s_alpha[col] = a;
+          s_point[col] = 0;
+          if (some) {
+            p.iters[v] = 0;
+            p.conv[v] = 1;
+            pp.alpha[v] = 0.0;
+          }
+        }
+      }
+      __syncwarp();
+    }
+    if (refilled && exhausted) {
+      const unsigned cols = columns(vid[0] >= 0, vid[1] >= 0);
+      if (__popc(cols) <= park_at) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          if (vid[j] < 0) continue;
+          const int64_t v = vid[j];
+          const int col = 2 * q + j;
+#pragma unroll
+          for (int mt = 0; mt < MT; ++mt) {
+            const int row = 8 * mt + g;
+            pp.Xp[v * KP + row] = x[mt][j];
+            pp.Yp[v * KP + row] = ybuf[row * 8 + col];
+          }
+          if (g == 0) {
+            const unsigned long long slot = atomicAdd(pp.n_park, 1ull);
+            pp.park[slot] = PathPark{s_best[col], static_cast<int>(v), s_point[col], it[j], 0};
+          }
+        }
+        break;
+      }
+    }
+    if (!__any_sync(kFull, vid[0] >= 0 || vid[1] >= 0)) break;
+
+    double mom[2], dx2[2], xn2[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) mom[j] = vid[j] >= 0 ? p.mom[it[j]] : 0.0;
+    dmma_fista_step<MT, NONNEG>(sG, ybuf, bbuf, live, x, mom, thr, c, lane, dx2, xn2);
+
+    // ---- per-voxel stopping rule (fista.rs:115-127)
+    bool conv[2] = {false, false}, fin[2] = {false, false};
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      if (vid[j] < 0) continue;
+      it[j] += 1;
+      if (!(dx2[j] > tol2x4 * fmax(xn2[j], 1e-24))) conv[j] = sqrt(dx2[j]) / fmax(sqrt(xn2[j]), 1e-12) < p.tol;
+      fin[j] = conv[j] || it[j] >= p.max_iter;
+    }
+    __syncwarp();
+    if (!__any_sync(kFull, fin[0] || fin[1])) continue;
+
+    // ---- finished points: residual, selection, next alpha
+    for (unsigned cols = columns(fin[0], fin[1]); cols != 0; cols &= cols - 1) {
+      const int col = __ffs(static_cast<int>(cols)) - 1, odd = col & 1;
+      const bool own = q == (col >> 1);
+      const int64_t v = __shfl_sync(kFull, odd ? vid[1] : vid[0], col >> 1);
+      int nnz = 0;  // its non-zero coefficients, in increasing row
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt) {
+        const double xv = odd ? x[mt][1] : x[mt][0];
+        const bool e = own && xv != 0.0;
+        const unsigned m = __ballot_sync(kFull, e);
+        if (e) {
+          const int pos = nnz + __popc(m & ((1u << lane) - 1u));
+          lval[pos] = xv;
+          lrow[pos] = 8 * mt + g;
+        }
+        nnz += __popc(m);
+      }
+      __syncwarp();
+      const float* sig = pp.sig ? pp.sig + v * pp.N : pp.data + pp.vox[v] * pp.N;
+      const double resid =
+          sqrt(sparse_rss<1>(sig, pp.Mt, pp.N, lval, lrow, nnz, lane));
+      const double limit = pp.mode == 3 ? (1.0 + pp.slack) * pp.rss_l2[v] : 0.0;
+      const int point = s_point[col];
+      double best = s_best[col];
+      const double a = s_alpha[col];
+      bool last = point + 1 >= pp.n_alphas;
+      const bool better = path_better(pp.mode, pp.N, nnz, resid * resid, limit, best, last);
+      const double next = last ? 0.0 : path_alpha(pp.amax[v], point + 1, pp.n_alphas, pp.eps);
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        if (!own || j != odd) continue;
+        if (better) {
+#pragma unroll
+          for (int mt = 0; mt < MT; ++mt) p.X[v * KP + 8 * mt + g] = x[mt][j];
+        }
+        if (g == 0) {
+          executed += it[j];
+          if (better) {
+            p.iters[v] = static_cast<uint32_t>(it[j]);
+            p.conv[v] = conv[j] ? 1 : 0;
+            pp.alpha[v] = a;
+            s_best[col] = best;
+          }
+          s_point[col] = point + 1;
+          s_alpha[col] = next;
+        }
+        need[j] = last;
+        if (last) vid[j] = -1;
+        it[j] = 0;
+        thr[j] = last ? INFINITY : __dmul_rn(p.step, next);
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) ybuf[(8 * mt + g) * 8 + col] = x[mt][j];  // y = x
+      }
+      __syncwarp();
+    }
+    live[0] = kFull;
+  }
+  if (p.iter_total) {
+    for (int o = 16; o > 0; o >>= 1) executed += __shfl_xor_sync(kFull, executed, o);
+    if (lane == 0) atomicAdd(p.iter_total, static_cast<unsigned long long>(executed));
+  }
+}
+
 }  // namespace csd

@@ -64,3 +64,27 @@ def test_order_8_two_voxels_per_warp_equal_one(v, oracle):
     num = np.linalg.norm(one["coef64"] - ref["coef64"], axis=1)
     assert (num <= 1e-5 * np.linalg.norm(ref["coef64"], axis=1)).all()
     assert np.abs(one["iterations"].astype(int) - ref["iterations"].astype(int)).max() <= 1
+
+
+@pytest.mark.parametrize("order,v", [(6, 5), (6, 2400), (6, 9475), (4, 9475), (8, 40)])
+@pytest.mark.parametrize("mode", ["l2-anchored", "path-bic"])
+def test_fused_path_equals_the_path_point_by_point(order, v, mode):
+    """Sizes of the fused path's three forms at order 6 (one and two voxels
+    per warp; from 9,472 the DMMA slots, which hand their last voxels over).
+    The residuals behind the selection are summed in another order (relative
+    1e-15), so a selection within that of a tie could differ; none does here.
+    """
+    from cs_dmri_b200 import _abi
+    ph, data, mask = tiled(v)
+    kw = dict(radial_order=order, alpha_mode=mode, path_n_alphas=9)
+    fused = fit(ph, data, mask, **kw)
+    _abi.set_option(_abi.OPT_FISTA_SHAPE, 16)  # a forced shape walks the path point by point
+    try:
+        walk = fit(ph, data, mask, **kw)
+    finally:
+        _abi.set_option(_abi.OPT_FISTA_SHAPE, 0)
+    for k in KEYS + ("alpha",):
+        np.testing.assert_array_equal(fused[k], walk[k])
+    for k in ("bic", "r2", "residual_l2"):
+        np.testing.assert_allclose(fused[k], walk[k], rtol=1e-6, atol=1e-6)
+    assert fused["total_iterations"] == walk["total_iterations"]
