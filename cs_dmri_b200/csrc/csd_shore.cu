@@ -33,6 +33,7 @@
 #include <mutex>
 #include <string>
 #include <thread>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/csd_shore.h"
@@ -836,7 +837,7 @@ void launch_fista_sparse_p(csd_handle* h, const csd::FistaParams& p) {
 // CSD_OPT_FISTA_SHAPE left at 0; every kernel computes the same iterates).
 // Measured per volume fit on B200, sparse against k_fista_v3, N = 259:
 //   order 4:   74,088 voxels 1.85 / 1.94 ms, 300,763 voxels 6.41 / 5.25 ms
-//   order 6:    4,000 voxels 0.99 / 2.80 ms, 74,088 voxels 4.29 / 4.32 ms,
+//   order 6:    4,000 voxels 0.84 / 2.80 ms, 74,088 voxels 4.29 / 4.32 ms,
 //             125,000 voxels 6.97 / 6.25 ms
 //   order 8:   32,000 voxels 4.56 / 6.87 ms, 300,763 voxels 33.2 / 47.5 ms
 // A warp of k_fista_v3 takes 2 us an iteration for its eight voxels and the
@@ -852,12 +853,12 @@ bool sparse_fista(const csd_handle* h, int64_t n_work) {
 }
 
 // One voxel per warp has the shorter iteration, two share the reads of G's
-// columns (per voxel-iteration 85 against 72 wavefronts at order 6): two from
-// about twice the voxels that one per warp holds at once (order 6: 4,000
-// voxels 0.99 / 1.06 ms, 16,384 voxels 1.57 / 1.54 ms, 64,000 voxels 4.07 /
-// 3.77 ms; order 8: 8,000 voxels 1.56 / 1.80 ms, 16,000 voxels 2.43 / 2.40
-// ms).  At order 4 one is faster at every size measured (64,000 voxels 1.69 /
-// 1.78 ms).
+// columns (per voxel-iteration 100 against 72 wavefronts at order 6): two
+// from about four times the voxels that one per warp holds at once (order 6:
+// 4,000 voxels 0.84 / 1.06 ms, 16,384 voxels 1.57 / 1.54 ms, 64,000 voxels
+// 4.07 / 3.77 ms; order 8: 8,000 voxels 1.56 / 1.80 ms, 16,000 voxels 2.43 /
+// 2.40 ms).  At order 4 one is faster at every size measured (64,000 voxels
+// 1.69 / 1.78 ms).
 void launch_fista_sparse(csd_handle* h, const csd::FistaParams& p) {
   switch (h->K) {
     case 29: launch_fista_sparse_p<29, 1, 16, 2>(h, p); break;
@@ -865,7 +866,7 @@ void launch_fista_sparse(csd_handle* h, const csd::FistaParams& p) {
       if (p.n_work > 64 * h->num_sms)
         launch_fista_sparse_p<72, 2, 16, 1>(h, p);
       else
-        launch_fista_sparse_p<72, 1, 16, 2>(h, p);
+        launch_fista_sparse_p<72, 1, 16, 1>(h, p);
       break;
     case 145:
       if (p.n_work > 96 * h->num_sms)
@@ -969,7 +970,7 @@ void launch_path_fused(csd_handle* h, const csd::PathParams& p0) {
       if (!p.resume && V > 16 * h->num_sms)
         launch_path_sparse_p<72, 2, 16, 1>(h, p);
       else
-        launch_path_sparse_p<72, 1, 16, 2>(h, p);
+        launch_path_sparse_p<72, 1, 16, 1>(h, p);
       break;
     case 145: launch_path_sparse_p<145, 1, 16, 1>(h, p); break;
     default: throw Error{CSD_ERR_INVALID, "the fused alpha path is built for radial orders 4, 6 and 8"};

@@ -13,10 +13,12 @@
 // order 6: 100 wavefronts of 128 B a voxel-iteration, 85 % of the pipe's
 // rate; two per warp read each column of their common list once: 72, at 65 %
 // with the issue slots at 63 %); for a few voxels the latency of one
-// iteration, 0.3 us against the 1.25-2 us of a DMMA warp.  Volume fits, N =
-// 259, against the DMMA kernel alone: 108 voxels 1.64 -> 0.47 ms, 4,000
-// voxels 3.55 -> 0.99 ms, 32,000 voxels at order 8 11.4 -> 3.5 ms (with the
-// residual pass that no output reads dropped there).
+// iteration, 0.5-0.6 us against the 1.25-2 us of a DMMA warp.  An SM partition
+// takes 32 B a cycle from shared memory, broadcasts included, so a column
+// costs its warp 18 cycles at order 6 and 36 at order 8 besides 12 for its
+// list entry.  Volume fits, N = 259, against the DMMA kernel alone: 108 voxels
+// 1.64 -> 0.42 ms, 4,000 voxels 3.55 -> 0.84 ms, 32,000 voxels at order 8
+// 11.4 -> 3.5 ms (with the residual pass that no output reads dropped there).
 #pragma once
 
 #include <cstdint>
@@ -82,7 +84,12 @@ struct SparseShape {
 
 // The states of a warp's P voxel slots and one FISTA iteration of them all
 // (src/solver/fista.rs:89-128).
-template <int K, int P, bool NONNEG>
+// WIDE: groups of eight columns while more than four are left (a group's chain
+// is two shared-memory latencies and its dependent FMAs, so fewer, wider groups
+// shorten an iteration where registers allow: 4,000 voxels at order 6, 128
+// registers and 16 warps per SM, 0.84 ms; groups of four, 64 registers and 32
+// warps, 0.99 ms).
+template <int K, int P, bool NONNEG, bool WIDE>
 struct SparseFista {
   using S = SparseShape<K, P>;
   double x[P][S::NR], y[P][S::NR], b[P][S::NR];
@@ -102,11 +109,17 @@ struct SparseFista {
       const int j = e / S::LD, r = e - j * S::LD;
       g[e] = r < K ? __ldg(G + j * S::KP + r) : 0.0;
     }
-    lane = threadIdx.x & 31;
-    const uint32_t base = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
+    attach(g, smem + S::G_BYTES + (threadIdx.x >> 5) * S::WARP_BYTES, threadIdx.x & 31);
+  }
+
+  // The warp's states over a matrix already in shared memory (columns of
+  // stride LD) and its list (WARP_BYTES), every slot empty.
+  __device__ __forceinline__ void attach(const double* g, void* list, int l) {
+    lane = l;
+    const uint32_t base = static_cast<uint32_t>(__cvta_generic_to_shared(g));
     gp = base + 16u * lane;
     gr = base + 8u * (64 * S::PAIRS + (lane < S::REM ? lane : 0));
-    lv = base + static_cast<uint32_t>(S::G_BYTES + (threadIdx.x >> 5) * S::WARP_BYTES);
+    lv = static_cast<uint32_t>(__cvta_generic_to_shared(list));
     li = lv + static_cast<uint32_t>(P * sizeof(double) * S::CAP);
 #pragma unroll
     for (int p = 0; p < P; ++p) clear(p);
@@ -133,6 +146,51 @@ struct SparseFista {
     else
       sp_st_2f64(lv + 16u * pos, y[0][i], y[P - 1][i], e);
     sp_st_s32(li + 4u * pos, row * static_cast<int>(sizeof(double) * S::LD), e);
+  }
+
+  static constexpr int U = P == 1 ? 4 : 2;  // columns per group
+
+  // acc += the C columns of list entries t .. t + C - 1.
+  template <int C>
+  __device__ __forceinline__ void group(int t, double (&acc)[P][S::NR]) const {
+    uint32_t off[C];
+    double yv[C][P];
+    if constexpr (C == 2) {
+      const int2 id = sp_ld_i2(li + 4u * t);
+      off[0] = id.x, off[1] = id.y;
+    } else {
+#pragma unroll
+      for (int c = 0; c < C; c += 4) {
+        const int4 id = sp_ld_i4(li + 4u * (t + c));
+        off[c] = id.x, off[c + 1] = id.y, off[c + 2] = id.z, off[c + 3] = id.w;
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < C * P; e += 2) {
+      const double2 v = sp_ld_v2(lv + 8u * (P * t + e));
+      yv[e / P][e % P] = v.x;
+      yv[(e + 1) / P][(e + 1) % P] = v.y;
+    }
+    double2 g2[C][S::PAIRS > 0 ? S::PAIRS : 1];
+    double g1[C];
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      g1[c] = 0.0;
+#pragma unroll
+      for (int i = 0; i < S::PAIRS; ++i) g2[c][i] = sp_ld_g2(gp + off[c] + 512u * i);
+      sp_ld_g1(g1[c], gr + off[c], lane < S::REM);
+    }
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+#pragma unroll
+      for (int p = 0; p < P; ++p) {
+#pragma unroll
+        for (int i = 0; i < S::PAIRS; ++i) {
+          acc[p][2 * i] = fma(g2[c][i].x, yv[c][p], acc[p][2 * i]);
+          acc[p][2 * i + 1] = fma(g2[c][i].y, yv[c][p], acc[p][2 * i + 1]);
+        }
+        acc[p][S::NR - 1] = fma(g1[c], yv[c][p], acc[p][S::NR - 1]);
+      }
   }
 
   // acc = G y for every slot.  The rows with a non-zero y in any slot are
@@ -163,7 +221,6 @@ struct SparseFista {
       list_row(64 * S::PAIRS + lane, S::NR - 1, e, n + __popc(me & lt));
       n += __popc(me);
     }
-    constexpr int U = P == 1 ? 4 : 2;  // columns per group
     {
       const bool pad = lane < U - 1;
       if constexpr (P == 1)
@@ -177,46 +234,12 @@ struct SparseFista {
     for (int p = 0; p < P; ++p)
 #pragma unroll
       for (int i = 0; i < S::NR; ++i) acc[p][i] = 0.0;
-    double g1[U];
-#pragma unroll
-    for (int c = 0; c < U; ++c) g1[c] = 0.0;
-    const bool rem = lane < S::REM;
+    int t = 0;
+    if constexpr (WIDE)
 #pragma unroll 1
-    for (int t = 0; t < n; t += U) {
-      uint32_t off[U];
-      double yv[U][P];
-      if constexpr (U == 4) {
-        const int4 id = sp_ld_i4(li + 4u * t);
-        off[0] = id.x, off[1] = id.y, off[2] = id.z, off[3] = id.w;
-      } else {
-        const int2 id = sp_ld_i2(li + 4u * t);
-        off[0] = id.x, off[1] = id.y;
-      }
-#pragma unroll
-      for (int e = 0; e < U * P; e += 2) {
-        const double2 v = sp_ld_v2(lv + 8u * (P * t + e));
-        yv[e / P][e % P] = v.x;
-        yv[(e + 1) / P][(e + 1) % P] = v.y;
-      }
-      double2 g2[U][S::PAIRS > 0 ? S::PAIRS : 1];
-#pragma unroll
-      for (int c = 0; c < U; ++c) {
-#pragma unroll
-        for (int i = 0; i < S::PAIRS; ++i) g2[c][i] = sp_ld_g2(gp + off[c] + 512u * i);
-        sp_ld_g1(g1[c], gr + off[c], rem);
-      }
-#pragma unroll
-      for (int c = 0; c < U; ++c)
-#pragma unroll
-        for (int p = 0; p < P; ++p) {
-#pragma unroll
-          for (int i = 0; i < S::PAIRS; ++i) {
-            acc[p][2 * i] = fma(g2[c][i].x, yv[c][p], acc[p][2 * i]);
-            acc[p][2 * i + 1] = fma(g2[c][i].y, yv[c][p], acc[p][2 * i + 1]);
-          }
-          acc[p][S::NR - 1] = fma(g1[c], yv[c][p], acc[p][S::NR - 1]);
-        }
-    }
+      for (; n - t > 4; t += 8) group<8>(t, acc);
+#pragma unroll 1
+    for (; t < n; t += U) group<U>(t, acc);
     __syncwarp();
   }
 
@@ -263,8 +286,9 @@ struct SparseFista {
 template <int K, int P, int MAXWARPS, int MINCTAS, bool NONNEG>
 __global__ void __launch_bounds__(32 * MAXWARPS, MINCTAS) k_fista_sparse(FistaParams p) {
   using S = SparseShape<K, P>;
+  constexpr bool WIDE = P == 1 && K == 72;
   extern __shared__ __align__(16) unsigned char sp_smem[];
-  SparseFista<K, P, NONNEG> f;
+  SparseFista<K, P, NONNEG, WIDE> f;
   f.init(p.G, sp_smem);
   __syncthreads();
   const unsigned long long n_work = p.n_work_dev ? *p.n_work_dev : static_cast<unsigned long long>(p.n_work);
@@ -442,7 +466,7 @@ __global__ void __launch_bounds__(32 * MAXWARPS, MINCTAS) k_path_sparse(PathPara
   using S = SparseShape<K, P>;
   extern __shared__ __align__(16) unsigned char sp_smem[];
   const FistaParams& p = q.f;
-  SparseFista<K, P, NONNEG> f;
+  SparseFista<K, P, NONNEG, (P == 1 && K == 72)> f;
   f.init(p.G, sp_smem);
   __syncthreads();
   const double c = p.step * p.n_inv;
