@@ -18,10 +18,25 @@
 //      two triangles of 8 x 8 tiles of the upper triangle in registers
 //      (GramPlan); b_v = M_v^T s_v alongside;
 //   3. lambda_max(G_v) by Lanczos (a fixed number of steps, the largest Ritz
-//      value by multisection of the tridiagonal's Sturm count, one point per
-//      thread);
-//   4. FISTA in the Gram form with G_v in shared memory (one thread per row of
-//      the product, 16-byte loads), the reference's update and stopping rule.
+//      value by multisection of the tridiagonal's spectrum, one point per
+//      thread); its products split G_v's columns and rows over the warps;
+//   4. FISTA in the Gram form on one warp, G_v in shared memory: y has 9 % of
+//      its entries non-zero at order 8, so the listed columns alone are added
+//      (SparseFista), with no barrier in an iteration.
+//
+// What bounds it: latency, one voxel at a time per SM (two CTAs at order 6; G_v
+// takes 169 KB at order 8).  SM cycles per voxel at order 8, reference rule,
+// ~145 iterations: Gram step 112 k (~50 k of it the DMMA pipe's floor), Lanczos
+// 155 k (40 steps of ~3.4 k and ~18 k for the tridiagonal's eigenvalue; one
+// thread per row of the product and a Sturm count with a division a step took
+// 253 k), FISTA 191 k (1.3 k an iteration; spread over the CTA with three
+// barriers it took 3.4 k).  12,288 voxels at order 8: reference rule 38.5 ->
+// 19.9 ms; order 6 33.9 -> 14.5 ms; certified modes, 20,000 voxels: FP64
+// 20.0 -> 16.0 and 14.8 -> 10.9 ms, mixed 18.0 -> 16.1 and 12.2 -> 10.5 ms.
+// Tried: the products from the Gram step's accumulator tiles while in
+// registers, each off-diagonal tile for both halves (3.0 k cycles a product,
+// most of it shuffles), and the recurrence's vectors on one warp (2.5 k a
+// step against 1.0 k).
 #pragma once
 
 namespace csd {
@@ -79,8 +94,8 @@ struct GraddevParams {
 // padding columns) and NSH SH values (row stride YS); both strides are odd,
 // so the fragment loads of four consecutive rows fall in distinct banks.
 struct GdLayout {
-  int K, Kp, LDG, LDF, NL, NSH, RS, YS, LC;
-  size_t g, vec, red, tri, tab, rows, colmap, nzv, nzi, total_bytes;
+  int K, Kp, LDG, LDF, NL, NSH, RS, YS, list_cap;
+  size_t g, vec, red, tri, tab, rows, colmap, list, total_bytes;
   __host__ __device__ GdLayout(int K_, int radial_order, int N) {
     K = K_;
     Kp = 8 * ((K + 7) / 8);
@@ -105,12 +120,10 @@ struct GdLayout {
     tab = tri + 128;                                         // kappa per (n, l), SH norm per (l, k)
     rows = tab + ((static_cast<size_t>(NL + NSH) + 1) & ~static_cast<size_t>(1));  // N ints
     colmap = rows + (static_cast<size_t>(N) + 1) / 2;        // column map (ints)
-    // FISTA's nonzero entries of y, one list per partial sum of the product
-    // (gd_gemv_nz): values (doubles) and indices (ints), LC slots each
-    LC = (K + 3) / 4 + 4;
-    nzv = colmap + (static_cast<size_t>(K) + 1) / 2;
-    nzi = nzv + 4 * static_cast<size_t>(LC);
-    total_bytes = 8 * (nzi + 2 * static_cast<size_t>(LC) + 2);
+    // FISTA's non-zero entries of y: values, then byte offsets of their columns
+    list_cap = (K + 3) / 4 * 4 + 4;
+    list = (colmap + (static_cast<size_t>(K) + 1) / 2 + 1) & ~static_cast<size_t>(1);
+    total_bytes = 8 * (list + static_cast<size_t>(list_cap) + list_cap / 2 + 2);
   }
 };
 
@@ -128,8 +141,8 @@ __device__ __forceinline__ double gd_block_sum(double a, double* red) {
   return s;
 }
 
-// The same sum into slots no thread reads any more, so without the barrier
-// before the write: the caller separates the reads of an earlier sum into
+// The same sum (eight warps) into slots no thread reads any more, so without
+// the barrier before the write: the caller separates the reads of an earlier sum into
 // `slots` from this write by a barrier of its own.
 __device__ __forceinline__ double gd_block_sum_fresh(double a, double* slots) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -137,90 +150,61 @@ __device__ __forceinline__ double gd_block_sum_fresh(double a, double* slots) {
   for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(kFull, a, o);
   if (lane == 0) slots[warp] = a;
   __syncthreads();
-  double s = 0.0;
-  for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) s += slots[w];
-  return s;
+  return ((slots[0] + slots[1]) + (slots[2] + slots[3])) + ((slots[4] + slots[5]) + (slots[6] + slots[7]));
 }
 
-// out[i] = sum_j G[i][j] v[j] for i < K, one thread per row: 16-byte loads of
-// G's row and of v (both in shared memory), four per step, into four
-// independent partial sums added at the end.
-__device__ __forceinline__ void gd_gemv(const double* G, int LDG, int K, const double* v, double* out) {
-  for (int i = threadIdx.x; i < K; i += blockDim.x) {
-    const double2* gr = reinterpret_cast<const double2*>(G + static_cast<size_t>(i) * LDG);
-    const double2* v2 = reinterpret_cast<const double2*>(v);
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-    const int h = K >> 1;
-    int j = 0;
-    for (; j + 3 < h; j += 4) {  // eight loads in flight per step
-      const double2 g0 = gr[j], g1 = gr[j + 1], g2 = gr[j + 2], g3 = gr[j + 3];
-      const double2 w0 = v2[j], w1 = v2[j + 1], w2 = v2[j + 2], w3 = v2[j + 3];
-      a0 = fma(g0.x, w0.x, a0);
-      a1 = fma(g0.y, w0.y, a1);
-      a2 = fma(g1.x, w1.x, a2);
-      a3 = fma(g1.y, w1.y, a3);
-      a0 = fma(g2.x, w2.x, a0);
-      a1 = fma(g2.y, w2.y, a1);
-      a2 = fma(g3.x, w3.x, a2);
-      a3 = fma(g3.y, w3.y, a3);
-    }
-    for (; j < h; ++j) {
-      const double2 g0 = gr[j], w0 = v2[j];
-      a0 = fma(g0.x, w0.x, a0);
-      a1 = fma(g0.y, w0.y, a1);
-    }
-    if (K & 1) a2 = fma(G[static_cast<size_t>(i) * LDG + K - 1], v[K - 1], a2);
-    out[i] = (a0 + a1) + (a2 + a3);
+// The support iterations of the mixed mode on one warp: `iters` FISTA steps in
+// FP32 on G_v's hi plane (row stride LDF), products over the non-zero entries
+// of y only; row lane + 32 i of each vector in register i.  The list holds
+// K + 4 (value, row offset) pairs.
+template <int NR>
+__device__ __forceinline__ void gd_fista32(const float* G, int LDF, int K, const double* b64, float2* list,
+                                           const double* mom_tab, int iters, float c, float thr, int non_negative,
+                                           int lane, float (&x)[NR]) {
+  float y[NR], b[NR];
+#pragma unroll
+  for (int i = 0; i < NR; ++i) {
+    x[i] = y[i] = 0.f;
+    b[i] = lane + 32 * i < K ? static_cast<float>(b64[lane + 32 * i]) : 0.f;
   }
-}
-
-// Which of gd_gemv's four partial sums takes entry e: e mod 4 in its main
-// loop, e mod 2 in the remainder loop, the third for the last of an odd K.
-__device__ __forceinline__ int gd_gemv_sum_of(int e, int K) {
-  const int h = K >> 1, main = 8 * (h / 4);
-  return e < main ? (e & 3) : (e < 2 * h ? (e & 1) : 2);
-}
-
-// gd_gemv for a vector with few nonzeros: `cnt[r]` entries of sum r are
-// listed, in increasing index, as (nzi[r LC + k], nzv[r LC + k]).  Each sum
-// adds the same products in the same order as gd_gemv's, without the zero
-// ones (an exact product of zero leaves a sum unchanged: a sum that starts
-// at +0 never becomes -0), so the result is bit for bit gd_gemv's.
-__device__ __forceinline__ void gd_gemv_nz(const double* G, int LDG, int K, const int* cnt, const double* nzv,
-                                           const int* nzi, int LC, double* out) {
-  for (int i = threadIdx.x; i < K; i += blockDim.x) {
-    const double* gr = G + static_cast<size_t>(i) * LDG;
-    const int n0 = cnt[0], n1 = cnt[1], n2 = cnt[2], n3 = cnt[3];
-    const int nmax = max(max(n0, n1), max(n2, n3));
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-    for (int k = 0; k < nmax; ++k) {
-      if (k < n0) a0 = fma(gr[nzi[k]], nzv[k], a0);
-      if (k < n1) a1 = fma(gr[nzi[LC + k]], nzv[LC + k], a1);
-      if (k < n2) a2 = fma(gr[nzi[2 * LC + k]], nzv[2 * LC + k], a2);
-      if (k < n3) a3 = fma(gr[nzi[3 * LC + k]], nzv[3 * LC + k], a3);
+  const unsigned lt = (1u << lane) - 1u;
+  for (int it = 0; it < iters; ++it) {
+    const float mom = static_cast<float>(__ldg(mom_tab + it));
+    int n = 0;
+#pragma unroll
+    for (int i = 0; i < NR; ++i) {
+      const bool e = y[i] != 0.f;
+      const unsigned m = __ballot_sync(kFull, e);
+      if (e) list[n + __popc(m & lt)] = make_float2(y[i], __int_as_float((lane + 32 * i) * LDF));
+      n += __popc(m);
     }
-    out[i] = (a0 + a1) + (a2 + a3);
-  }
-}
-
-// The same product with FP32 entries, vector and sums: G_v's hi plane (row
-// stride LDF), four entries per 16-byte load.
-__device__ __forceinline__ void gd_gemv32(const float* G, int LDF, int K, const float* v, float* out) {
-  for (int i = threadIdx.x; i < K; i += blockDim.x) {
-    const float4* gr = reinterpret_cast<const float4*>(G + static_cast<size_t>(i) * LDF);
-    const float4* v4 = reinterpret_cast<const float4*>(v);
-    float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-    const int h = K >> 2;
-#pragma unroll 4
-    for (int j = 0; j < h; ++j) {
-      const float4 g = gr[j], w = v4[j];
-      a0 = fmaf(g.x, w.x, a0);
-      a1 = fmaf(g.y, w.y, a1);
-      a2 = fmaf(g.z, w.z, a2);
-      a3 = fmaf(g.w, w.w, a3);
+    if (lane < 4) list[n + lane] = make_float2(0.f, 0.f);
+    __syncwarp();
+    float acc[NR];
+#pragma unroll
+    for (int i = 0; i < NR; ++i) acc[i] = 0.f;
+    for (int t = 0; t < n; t += 4) {
+      float2 e[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) e[u] = list[t + u];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float* col = G + __float_as_int(e[u].y) + lane;
+#pragma unroll
+        for (int i = 0; i < NR; ++i)
+          if (lane + 32 * i < K) acc[i] = fmaf(col[32 * i], e[u].x, acc[i]);
+      }
     }
-    for (int j = 4 * h; j < K; ++j) a0 = fmaf(G[static_cast<size_t>(i) * LDF + j], v[j], a0);
-    out[i] = (a0 + a1) + (a2 + a3);
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < NR; ++i) {
+      if (lane + 32 * i >= K) continue;
+      const float cand = fmaf(-c, acc[i] - b[i], y[i]);
+      float xn = cand > thr ? cand - thr : (cand < -thr ? cand + thr : 0.f);
+      if (non_negative) xn = fmaxf(xn, 0.f);
+      y[i] = fmaf(mom, xn - x[i], xn);
+      x[i] = xn;
+    }
   }
 }
 
@@ -268,17 +252,21 @@ struct GramPlan {
   static_assert(NR <= 8 && TW >= 1 && TPT <= 2, "gram plan");
 };
 
-// Count of eigenvalues of the symmetric tridiagonal (a, b) below x (Sturm).
-__device__ __forceinline__ int sturm_below(const double* a, const double* b, int m, double x) {
-  int c = 0;
-  double d = a[0] - x;
-  if (d < 0.0) ++c;
+// Whether x lies above every eigenvalue of the symmetric tridiagonal (a, b):
+// the leading minors of x I - T, s_i = (x - a_i) s_{i-1} - b_{i-1}^2 s_{i-2},
+// are all positive.  b2 holds the squares; a and x are scaled to a spectrum
+// within [-1, 1], so 64 steps neither overflow nor underflow.  No division: the
+// Sturm quotients' chain of m divisions took 7 k cycles at m = 40, 84 k a voxel.
+__device__ __forceinline__ bool above_spectrum(const double* a, const double* b2, int m, double x) {
+  double s0 = 1.0, s1 = x - a[0];
+  bool ok = s1 > 0.0;
   for (int i = 1; i < m; ++i) {
-    const double dd = (d == 0.0) ? 1e-300 : d;
-    d = (a[i] - x) - b[i - 1] * b[i - 1] / dd;
-    if (d < 0.0) ++c;
+    const double s2 = fma(x - a[i], s1, -(b2[i - 1] * s0));
+    s0 = s1;
+    s1 = s2;
+    ok = ok && s2 > 0.0;
   }
-  return c;
+  return ok;
 }
 
 template <int MT>
@@ -306,14 +294,12 @@ __global__ void __launch_bounds__(256, (MT <= 9) ? 2 : 1) k_graddev_fit(GraddevP
   double* shn = kap + NL;                          // NSH: SH normalisation of (l, k)
   int* rows = reinterpret_cast<int*>(gd_smem + L.rows);
   int* col_map = reinterpret_cast<int*>(gd_smem + L.colmap);  // K: radial factor | SH entry << 16
-  double* nzv = gd_smem + L.nzv;                                // FISTA's nonzero y entries, by partial sum
-  int* nzi = reinterpret_cast<int*>(gd_smem + L.nzi);
-  __shared__ int gd_wcnt[8][4];  // per warp and partial sum: nonzero y entries
-  __shared__ int gd_ncnt[4];     // per partial sum
+  constexpr int KT_ = MT > 9 ? 145 : 72;                        // = K: the orders the host admits
   __shared__ int64_t s_v;
   __shared__ int s_n;
   __shared__ double s_lmax;
   __shared__ int s_first;
+  __shared__ int s_it, s_conv, s_above[8];
   __shared__ uint16_t gd_tri[kTriTable];  // (row, col) of a packed triangle, for the polish
   __shared__ double gd_rcp[kGdRcp];       // 1 / i: the recurrences' divisors as products
   for (int i = threadIdx.x; i < kGdRcp; i += blockDim.x) gd_rcp[i] = i > 0 ? 1.0 / i : 0.0;
@@ -648,54 +634,78 @@ __global__ void __launch_bounds__(256, (MT <= 9) ? 2 : 1) k_graddev_fit(GraddevP
     // ---- 3. lambda_max(G) by Lanczos: `steps` steps, the largest Ritz value
     // left in s_lmax (a lower bound of lambda_max, exact to ~1e-12 at 40)
     const int LDG = L.LDG;
-    // the FP64 product with G_v (from its planes in the mixed mode)
-    auto gemv64 = [&](const double* vin, double* vout) {
-      if (mixed)
-        gd_gemv_hl(Ghi, Glo, LDF, K, vin, vout);
-      else
-        gd_gemv(G, LDG, K, vin, vout);
+    // Lanczos step's G v: two warps to a quarter of the columns, one per half of
+    // the rows (16-byte loads, conflict-free; the heavier second halves on
+    // alternating partitions), so the matrix reads spread over the SM's four
+    // partitions, each of which takes 32 B a cycle; slot c of the vectors FISTA
+    // uses later (vx, vy, vgy, w) takes quarter c's sums.  T is double on G, or
+    // float on the hi plane with v in v32.
+    auto slot_of = [&](int s) -> double* { return s < 3 ? vx + s * Kp : lw; };
+    float* v32 = reinterpret_cast<float*>(gd_smem + L.list);
+    auto split_product = [&](auto type, const auto* Gm, int ld, const auto* vin) {
+      using T = decltype(type);
+      using T2 = std::conditional_t<std::is_same_v<T, double>, double2, float2>;
+      constexpr int QC = (KT_ + 3) / 4;                    // columns per quarter
+      constexpr int HALF = KT_ > 128 ? 64 : KT_ / 2;       // rows of the first half
+      constexpr int PAIRS = KT_ > 128 ? 32 : HALF / 2;     // lanes with a row pair
+      constexpr int REM = KT_ > 128 ? KT_ - 128 : 0;       // rows past both halves, on the second's warps
+      static_assert(HALF % 2 == 0 && 2 * HALF + REM == KT_, "row halves");
+      const int cq = warp >> 1, h = (warp ^ (warp >> 2)) & 1;
+      const int c0 = cq * QC, c1 = min(KT_, c0 + QC);
+      const T* gp = Gm + HALF * h + 2 * (lane < PAIRS ? lane : 0);
+      const T* gr = Gm + 2 * HALF + (lane < REM ? lane : 0);
+      T a0 = 0, a1 = 0, ar = 0;
+#pragma unroll 6
+      for (int c = c0; c < c1; ++c) {
+        const T vc = vin[c];
+        const T2 gv = *reinterpret_cast<const T2*>(gp + c * ld);
+        a0 = gv.x * vc + a0;
+        a1 = gv.y * vc + a1;
+        if (REM > 0 && h == 1) ar = gr[c * ld] * vc + ar;
+      }
+      double* s = slot_of(cq);
+      if (lane < PAIRS) *reinterpret_cast<double2*>(s + HALF * h + 2 * lane) = make_double2(a0, a1);
+      if (REM > 0 && h == 1 && lane < REM) s[2 * HALF + lane] = ar;
     };
-    // `lowp`: the vectors are FP32 (in the same slots) and the product uses
-    // G_v's hi plane; the sums and the tridiagonal stay FP64
+    // `lowp`: the products in FP32 on the hi plane; the vectors, the sums and
+    // the tridiagonal stay FP64
     auto run_lanczos = [&](int steps, bool lowp) {
       const int m = min(K, steps);
-      float* lv32 = reinterpret_cast<float*>(lv);
-      float* lvp32 = reinterpret_cast<float*>(lv_prev);
-      float* lw32 = reinterpret_cast<float*>(lw);
-      auto get = [&](const double* d, const float* f, int i) -> double {
-        return lowp ? static_cast<double>(f[i]) : d[i];
-      };
-      auto set = [&](double* d, float* f, int i, double x) {
-        if (lowp)
-          f[i] = static_cast<float>(x);
-        else
-          d[i] = x;
-      };
       for (int i = tid; i < Kp; i += blockDim.x) {
-        set(lv, lv32, i, (i < K) ? 1.0 + 0.5 * sin(1.7 * i + 0.3) : 0.0);  // fixed start vector
-        set(lv_prev, lvp32, i, 0.0);
+        lv[i] = (i < K) ? 1.0 + 0.5 * sin(1.7 * i + 0.3) : 0.0;  // fixed start vector
+        lv_prev[i] = 0.0;
       }
       {
-        const double e = (tid < K) ? get(lv, lv32, tid) : 0.0;  // K <= blockDim.x
+        const double e = (tid < K) ? lv[tid] : 0.0;  // K <= blockDim.x
         const double inv = 1.0 / sqrt(gd_block_sum(e * e, red));
-        if (tid < K) set(lv, lv32, tid, get(lv, lv32, tid) * inv);
+        if (tid < K) lv[tid] *= inv;
+        if (tid < K) v32[tid] = static_cast<float>(lv[tid]);
       }
       __syncthreads();
       int msteps = m;
       double beta_prev = 0.0;
-      // three barriers a step: w_i, v_i and v_prev_i are this thread's own
-      // entries (one row of the product per thread), the two sums use slots
-      // 0-7 and 8-15 of `red` (each read before the step's last barrier), and
-      // the last barrier orders the new v before the next step's product
+      // w_i, v_i and v_prev_i are this thread's own entries; the two sums use
+      // slots 0-7 and 8-15 of `red` (each read before the step's last
+      // barrier), and the last barrier orders the new v before the next
+      // step's product
       for (int j = 0; j < m; ++j) {
-        if (lowp)
-          gd_gemv32(Ghi, LDF, K, lv32, lw32);
-        else
-          gemv64(lv, lw);
-        const double wi = (tid < K) ? get(lw, lw32, tid) : 0.0, vi = (tid < K) ? get(lv, lv32, tid) : 0.0;
+        double wi = 0.0;
+        if (mixed && !lowp) {
+          gd_gemv_hl(Ghi, Glo, LDF, K, lv, lw);
+          wi = (tid < K) ? lw[tid] : 0.0;
+        } else {
+          if (lowp)
+            split_product(0.f, Ghi, LDF, v32);
+          else
+            split_product(0.0, G, LDG, lv);
+          __syncthreads();
+          if (tid < K) wi = (vx[tid] + vx[Kp + tid]) + (vx[2 * Kp + tid] + lw[tid]);
+        }
+        const double vi = (tid < K) ? lv[tid] : 0.0;
         const double al = gd_block_sum_fresh(wi * vi, red);
-        const double wn = (tid < K) ? wi - al * vi - beta_prev * get(lv_prev, lvp32, tid) : 0.0;
-        const double bt = sqrt(gd_block_sum_fresh(wn * wn, red + 8));
+        const double wn = (tid < K) ? wi - al * vi - beta_prev * lv_prev[tid] : 0.0;
+        const double b2 = gd_block_sum_fresh(wn * wn, red + 8);
+        const double ib = rsqrt(b2), bt = b2 * ib;
         if (tid == 0) {
           ta[j] = al;
           tb[j] = bt;
@@ -705,8 +715,9 @@ __global__ void __launch_bounds__(256, (MT <= 9) ? 2 : 1) k_graddev_fit(GraddevP
           break;
         }
         if (tid < K) {
-          set(lv_prev, lvp32, tid, vi);
-          set(lv, lv32, tid, wn / bt);
+          lv_prev[tid] = vi;
+          lv[tid] = wn * ib;
+          if (lowp) v32[tid] = static_cast<float>(wn * ib);
         }
         beta_prev = bt;
         __syncthreads();
@@ -719,20 +730,32 @@ __global__ void __launch_bounds__(256, (MT <= 9) ? 2 : 1) k_graddev_fit(GraddevP
           lo = fmin(lo, ta[i] - r);
           hi = fmax(hi, ta[i] + r);
         }
-        const int P = blockDim.x;  // points lo + (hi - lo) (t + 1) / (P + 1)
-        for (int round = 0; round < 12 && hi - lo > 1e-16 * fmax(fabs(hi), fabs(lo)); ++round) {
-          if (tid == 0) s_first = P;
-          __syncthreads();
-          const double x = lo + (hi - lo) * (tid + 1) / (P + 1.0);
-          if (sturm_below(ta, tb, msteps, x) == msteps) atomicMin(&s_first, tid);  // x above every eigenvalue
-          __syncthreads();
-          const int first = s_first;  // the top eigenvalue lies in (x_{first-1}, x_first]
-          const double nlo = lo + (hi - lo) * first / (P + 1.0);
-          hi = lo + (hi - lo) * (first + 1) / (P + 1.0);
-          lo = nlo;
-          __syncthreads();
+        const double scale = fmax(fabs(lo), fabs(hi));  // the spectrum within [-1, 1]
+        __syncthreads();
+        if (scale > 0.0 && tid < msteps) {
+          ta[tid] /= scale;
+          tb[tid] = (tb[tid] / scale) * (tb[tid] / scale);
         }
-        if (tid == 0) s_lmax = 0.5 * (lo + hi);
+        __syncthreads();
+        if (scale > 0.0) {
+          lo /= scale;
+          hi /= scale;
+          const int P = blockDim.x;  // points lo + (hi - lo) (t + 1) / (P + 1)
+          for (int round = 0; round < 12 && hi - lo > 2.3e-16 * fmax(fabs(hi), fabs(lo)); ++round) {
+            const double x = lo + (hi - lo) * (tid + 1) / (P + 1.0);
+            const unsigned ok = __ballot_sync(kFull, above_spectrum(ta, tb, msteps, x));
+            if (lane == 0) s_above[warp] = ok ? 32 * warp + __ffs(static_cast<int>(ok)) - 1 : P;
+            __syncthreads();
+            int first = P;  // the top eigenvalue lies in (x_{first-1}, x_first]
+#pragma unroll
+            for (int w = 7; w >= 0; --w) first = s_above[w] < P ? s_above[w] : first;
+            const double nlo = lo + (hi - lo) * first / (P + 1.0);
+            hi = lo + (hi - lo) * (first + 1) / (P + 1.0);
+            lo = nlo;
+            __syncthreads();
+          }
+        }
+        if (tid == 0) s_lmax = scale > 0.0 ? 0.5 * (lo + hi) * scale : 0.5 * (lo + hi);
       }
       __syncthreads();
     };
@@ -748,149 +771,97 @@ __global__ void __launch_bounds__(256, (MT <= 9) ? 2 : 1) k_graddev_fit(GraddevP
     double step = (n > 0) ? 1.0 / (p.kkt ? lip * kGdKktLipMargin : lip) : 0.0;
     const double alpha_v = p.alpha_v ? p.alpha_v[v] : p.alpha;
     double thr = __dmul_rn(step, alpha_v);
-    // `max_it` iterations from zero, stopping early below `tol` (never with tol 0)
-    auto run_fista = [&](int max_it, double tol, bool& converged) -> int {
-      for (int i = tid; i < Kp; i += blockDim.x) {
-        vx[i] = 0.0;
-        vy[i] = 0.0;
+    // FISTA from zero on G_v and b_v, x into vx: warp 0 with the FP64 matrix
+    // (SparseFista), `max_it` iterations or below `tol` (never with tol 0)
+    auto fista_warp = [&](auto nonneg, int max_it, double tol, bool& conv_out) -> int {
+      using F = SparseFista<KT_, 1, decltype(nonneg)::value, (MT > 9)>;
+      F f;
+      f.attach(G, gd_smem + L.list, lane);
+#pragma unroll
+      for (int i = 0; i < F::S::NR; ++i) {
+        const int row = F::S::row(i, lane);
+        f.b[0][i] = row < K ? vb[row] : 0.0;
       }
-      __syncthreads();
-      int it = 0;
-      converged = false;
-      // tol 0 (a fixed iteration count) needs no stopping test: no reductions
-      const bool check = tol > 0.0;
-      // with the FP64 matrix the reference rule's product reads only y's
-      // nonzero entries, listed after each update (gd_gemv_nz; one more
-      // barrier a step).  Measured at 300k voxels: order 8 0.909 -> 0.828 s;
-      // the converged-optimum modes' 16-32 iterations from zero gained
-      // nothing at order 8 and lost 5 % at order 6, so they keep the dense one.
-      const bool sparse = !mixed && check && K > 96;
-      const int my_sum = (tid < K) ? gd_gemv_sum_of(tid, K) : 0;
-      unsigned bal[4] = {0u, 0u, 0u, 0u};
-      double yn = 0.0;
-      auto list_nonzeros = [&]() {  // after a barrier that follows the counts' writes
-        if (tid < K && yn != 0.0) {
-          const unsigned mine = my_sum == 0 ? bal[0] : (my_sum == 1 ? bal[1] : (my_sum == 2 ? bal[2] : bal[3]));
-          int off = __popc(mine & ((1u << lane) - 1u));
-          for (int w = 0; w < warp; ++w) off += gd_wcnt[w][my_sum];
-          nzi[my_sum * L.LC + off] = tid;
-          nzv[my_sum * L.LC + off] = yn;
-        }
-        if (tid < 4) {
-          int t = 0;
-          for (int w = 0; w < 8; ++w) t += gd_wcnt[w][tid];
-          gd_ncnt[tid] = t;
-        }
-      };
-      if (tid < 4) gd_ncnt[tid] = 0;  // y = 0
-      __syncthreads();
-      double mom_next = (max_it > 0) ? p.mom[0] : 0.0;
-      while (n > 0 && it < max_it) {
+      f.thr[0] = thr;
+      const double c = __dmul_rn(step, n_inv);
+      int k = 0;
+      conv_out = false;
+      double mom_next = max_it > 0 ? __ldg(p.mom) : 0.0;
+      while (k < max_it && !conv_out) {
         const double mom = mom_next;
-        if (it + 1 < max_it) mom_next = p.mom[it + 1];  // in flight during the product
-        if (sparse)
-          gd_gemv_nz(G, LDG, K, gd_ncnt, nzv, nzi, L.LC, vgy);
-        else
-          gemv64(vy, vgy);
-        __syncthreads();
+        if (k + 1 < max_it) mom_next = __ldg(p.mom + k + 1);
+        double prod[1][F::S::NR];
+        f.product(prod);
+        conv_out = f.update(0, prod[0], mom, c, tol);
+        ++k;
+      }
+#pragma unroll
+      for (int i = 0; i < F::S::NR; ++i) {
+        const int row = F::S::row(i, lane);
+        if (row < Kp) vx[row] = f.x[0][i];
+      }
+      return k;
+    };
+    // The same with the planes' matrix, spread over the CTA (the mixed mode's
+    // uncertified voxels): one thread per row of the product
+    auto fista_planes = [&](int max_it, double tol, bool& conv_out) -> int {
+      for (int i = tid; i < Kp; i += blockDim.x) vx[i] = vy[i] = 0.0;
+      __syncthreads();
+      const double c = __dmul_rn(step, n_inv);
+      int k = 0;
+      conv_out = false;
+      while (k < max_it) {
+        gd_gemv_hl(Ghi, Glo, LDF, K, vy, vgy);
         double dx2 = 0.0, xn2 = 0.0;
-        yn = 0.0;
-        if (tid < K) {
-          const int i = tid;
-          const double grad = __dmul_rn(__dsub_rn(vgy[i], vb[i]), n_inv);
-          const double cand = __dsub_rn(vy[i], __dmul_rn(step, grad));
-          double sv;
-          if (cand > thr)
-            sv = __dsub_rn(cand, thr);
-          else if (cand < -thr)
-            sv = __dadd_rn(cand, thr);
-          else
-            sv = 0.0;
-          const double xn = p.non_negative ? fmax(sv, 0.0) : sv;
-          const double d = __dsub_rn(xn, vx[i]);
-          yn = __dadd_rn(xn, __dmul_rn(mom, d));
-          vy[i] = yn;
-          vx[i] = xn;
-          dx2 = __dmul_rn(d, d);
-          xn2 = __dmul_rn(xn, xn);
+        if (tid < K) {  // vgy[tid] is this thread's own row
+          const double xn = p.non_negative ? fista_prox<true>(vgy[tid], vb[tid], vy[tid], c, thr)
+                                           : fista_prox<false>(vgy[tid], vb[tid], vy[tid], c, thr);
+          const double d = __dsub_rn(xn, vx[tid]);
+          lw[tid] = fma(p.mom[k], d, xn);
+          vx[tid] = xn;
+          dx2 = d * d;
+          xn2 = xn * xn;
         }
-        if (sparse) {
-          const bool nz = tid < K && yn != 0.0;
-#pragma unroll
-          for (int r = 0; r < 4; ++r) bal[r] = __ballot_sync(kFull, nz && my_sum == r);
-          if (lane < 4) gd_wcnt[warp][lane] = __popc(lane == 0 ? bal[0] : (lane == 1 ? bal[1] : (lane == 2 ? bal[2] : bal[3])));
-        }
-        if (!check) {
-          ++it;
-          __syncthreads();  // the new y before the next product
-          if (sparse) {
-            list_nonzeros();
-            __syncthreads();
-          }
-          continue;
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          dx2 += __shfl_xor_sync(kFull, dx2, o);
-          xn2 += __shfl_xor_sync(kFull, xn2, o);
-        }
-        if (lane == 0) {
-          red[2 * warp] = dx2;
-          red[2 * warp + 1] = xn2;
-        }
+        const double sdx = gd_block_sum(dx2, red), sxn = gd_block_sum(xn2, red);
+        if (tid < K) vy[tid] = lw[tid];
+        ++k;
         __syncthreads();
-        if (sparse) list_nonzeros();
-        double sdx = 0.0, sxn = 0.0;
-        for (int w = 0; w < 8; ++w) {
-          sdx += red[2 * w];
-          sxn += red[2 * w + 1];
-        }
-        ++it;
-        const double rel = sqrt(sdx) / fmax(sqrt(sxn), 1e-12);
-        // red is next written after the next iteration's first barrier, which
-        // every thread reaches only once it has read it; the lists need one
-        if (sparse) __syncthreads();
-        if (rel < tol) {
-          converged = true;
+        if (sqrt(sdx) / fmax(sqrt(sxn), 1e-12) < tol) {
+          conv_out = true;
           break;
         }
       }
-      __syncthreads();  // the polish reuses red and the vectors as scratch
-      return it;
+      return k;
     };
-    // the mixed mode's support iterations: the same update in FP32 on G_v's
-    // hi plane, a fixed count, x_i and b_i in the registers of thread i and y
-    // in FP32 in y's slot; x is left in FP64 in vx for the polish
-    auto run_fista32 = [&](int iters) -> int {
-      float* y32 = reinterpret_cast<float*>(vy);
-      float* gy32 = reinterpret_cast<float*>(vgy);
-      const float step32 = static_cast<float>(step), thr32 = static_cast<float>(thr);
-      const float ninv32 = static_cast<float>(n_inv);
-      const float bi = (tid < K) ? static_cast<float>(vb[tid]) : 0.f;
-      float xi = 0.f;
-      for (int i = tid; i < Kp; i += blockDim.x) y32[i] = 0.f;
-      __syncthreads();
-      double mom_next = (iters > 0) ? p.mom[0] : 0.0;
-      for (int it = 0; n > 0 && it < iters; ++it) {
-        const float mom = static_cast<float>(mom_next);
-        if (it + 1 < iters) mom_next = p.mom[it + 1];
-        gd_gemv32(Ghi, LDF, K, y32, gy32);
-        __syncthreads();
-        if (tid < K) {
-          const float grad = (gy32[tid] - bi) * ninv32;
-          const float cand = y32[tid] - step32 * grad;
-          float sv = 0.f;
-          if (cand > thr32)
-            sv = cand - thr32;
-          else if (cand < -thr32)
-            sv = cand + thr32;
-          const float xn = p.non_negative ? fmaxf(sv, 0.f) : sv;
-          y32[tid] = xn + mom * (xn - xi);
-          xi = xn;
+    // on warp 0 of the FP64 matrix, the result in s_it / s_conv after a barrier
+    auto run_fista = [&](int max_it, double tol, bool& conv_out) -> int {
+      if (warp == 0) {
+        bool cv = false;
+        const int k = n == 0 ? 0
+                      : p.non_negative ? fista_warp(std::true_type{}, max_it, tol, cv)
+                                       : fista_warp(std::false_type{}, max_it, tol, cv);
+        if (n == 0)
+          for (int i = lane; i < Kp; i += 32) vx[i] = 0.0;
+        if (lane == 0) {
+          s_it = k;
+          s_conv = cv ? 1 : 0;
         }
-        __syncthreads();  // the new y before the next product
       }
-      for (int i = tid; i < Kp; i += blockDim.x) vx[i] = (i == tid && i < K) ? static_cast<double>(xi) : 0.0;
+      __syncthreads();
+      conv_out = s_conv != 0;
+      return s_it;
+    };
+    // the mixed mode's support iterations, x left in FP64 in vx for the polish
+    auto run_fista32 = [&](int iters) -> int {
+      if (warp == 0) {
+        constexpr int NR = (KT_ + 31) / 32;
+        float xs[NR];
+        gd_fista32<NR>(Ghi, LDF, K, vb, reinterpret_cast<float2*>(gd_smem + L.list), p.mom, n > 0 ? iters : 0,
+                       static_cast<float>(step * n_inv), static_cast<float>(thr), p.non_negative, lane, xs);
+#pragma unroll
+        for (int i = 0; i < NR; ++i)
+          if (lane + 32 * i < Kp) vx[lane + 32 * i] = lane + 32 * i < K ? static_cast<double>(xs[i]) : 0.0;
+      }
       __syncthreads();
       return n > 0 ? iters : 0;
     };
@@ -950,7 +921,8 @@ __global__ void __launch_bounds__(256, (MT <= 9) ? 2 : 1) k_graddev_fit(GraddevP
         step = 1.0 / lip;
         thr = __dmul_rn(step, alpha_v);
         bool conv_ref = false;
-        it += run_fista(p.max_iter, p.tol, conv_ref);
+        it += mixed ? fista_planes(p.max_iter, p.tol, conv_ref) : run_fista(p.max_iter, p.tol, conv_ref);
+        __syncthreads();
       }
       converged = cert || n == 0;
       if (tid == 0) {
