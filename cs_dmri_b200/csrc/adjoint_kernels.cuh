@@ -249,74 +249,39 @@ __global__ void k_identity_rows(double* __restrict__ I, int K, int Kp) {
   if (i < K * Kp) I[i] = ((i % Kp) == (i / Kp)) ? 1.0 : 0.0;
 }
 
-// out[v][r] = sum over k < cols of At[k * rows + r] in[v][k]: a fixed matrix
-// A (rows x cols, stored transposed so that a warp's lanes read consecutive
-// rows) applied to every voxel's vector, FP64 with fused multiply-adds in
-// index order.  Eight voxels per warp: their inputs are staged in the warp's
-// shared slice as [k][voxel], so each coalesced load of a column of A feeds
-// eight FMAs with operands from four 16-byte broadcast reads.  Outputs in
-// FP64 and / or rounded to FP32 (each nullable).
-__global__ void __launch_bounds__(256) k_apply64(const double* __restrict__ At, int rows, int cols,
-                                                 const double* __restrict__ in, int64_t ldin, int64_t V,
-                                                 double* __restrict__ out, float* __restrict__ out32,
-                                                 int64_t ldout) {
-  extern __shared__ __align__(16) double apply_smem[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double* sI = apply_smem + static_cast<size_t>(warp) * 8 * cols;
-  const int64_t groups = (V + 7) / 8;
-  const int64_t nwarps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
-  for (int64_t g = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + warp; g < groups; g += nwarps) {
-    const int64_t v0 = 8 * g;
-    const int nv = V - v0 < 8 ? static_cast<int>(V - v0) : 8;
-    __syncwarp();
-    for (int j = 0; j < 8; ++j)
-      for (int k = lane; k < cols; k += 32) sI[k * 8 + j] = j < nv ? in[(v0 + j) * ldin + k] : 0.0;
-    __syncwarp();
-    const double2* sI2 = reinterpret_cast<const double2*>(sI);
-    for (int r = lane; r < rows; r += 32) {
-      double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-      for (int k = 0; k < cols; ++k) {
-        const double a = At[static_cast<size_t>(k) * rows + r];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const double2 xv = sI2[k * 4 + j];
-          acc[2 * j] = fma(a, xv.x, acc[2 * j]);
-          acc[2 * j + 1] = fma(a, xv.y, acc[2 * j + 1]);
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-        if (j < nv) {
-          if (out) out[(v0 + j) * ldout + r] = acc[j];
-          if (out32) out32[(v0 + j) * ldout + r] = static_cast<float>(acc[j]);
-        }
-    }
-  }
-}
-
-// The same product on the FP64 tensor cores, for a matrix that fits in
-// shared memory: A is staged once per persistent CTA in m8n8k4 A-fragment
-// order, frag[(mt * KT + kt) * 32 + lane] = A[8 mt + lane / 4][4 kt + lane % 4]
-// (zero padded; read from At), so each fragment is one conflict-free 256-byte
-// read.  A warp takes 8 voxels at a time: out^T (rows x 8) = A in^T, the
-// voxels' inputs as B fragments, reused across a chunk of kApplyMtc row tiles
-// held as accumulators.  The fragments come from global memory, so they are
-// fetched well ahead of their DMMAs: with KT <= kApplyKtr (inputs of up to 96
-// entries) a group's KT fragments sit in registers and serve every row
-// chunk, and the next group's are loaded while this one computes; longer
-// inputs stream through a ring of kApplyPf fragments.  Every tile accumulates
-// its k-steps in increasing order either way.
+// out[v][r] = sum over k < cols of At[k * lda + r] in[v][k]: a fixed matrix A
+// (rows x cols, stored transposed) applied to every voxel's vector on the FP64
+// tensor cores, outputs in FP64 and / or rounded to FP32 (each nullable; zeros
+// in rows .. rows_out).  A CTA stages a chunk of row tiles
+// of A (blockIdx.y; all of them when they fit) in m8n8k4 A-fragment order,
+// frag[(mt * KT + kt) * 32 + lane] = A[8 mt + lane / 4][4 kt + lane % 4] (zero
+// padded; read from At, row stride lda), so each fragment is one conflict-free
+// 256-byte read.  A warp takes 8 voxels at a time: out^T (rows x 8) = A in^T,
+// the voxels' inputs as B fragments shared by kApplyMtc row tiles held as
+// accumulators.  They come from global memory (row `idx[v]` of `in`, or row v)
+// through a ring of kApplyPf fragments, refilled in place as their DMMAs are
+// issued (a register move would wait for the load still in flight).  Every
+// tile accumulates its k-steps in increasing order: one FMA chain in index
+// order, as k_rhs.  With `add` (laid out as out, which it may be)
+// the output is add + sign A in.
+//
+// Chunks of row tiles: a matrix larger than one CTA's shared memory (the
+// order-8 ODF, adjoint and design products take 300-420 KB) ran on plain FMAs,
+// every warp streaming the matrix from L2: 310 us a product for 3,001 voxels
+// (362 x 145 and like), here 31 us.  A short batch also splits the rows
+// further, so that every SM has a chunk.
 constexpr int kApplyMtc = 12;
-constexpr int kApplyKtr = 24;
 constexpr int kApplyPf = 8;
+constexpr int kApplyWarps = 16;
 
-template <bool kRegs>
-__global__ void __launch_bounds__(256, 1) k_apply_dmma(const double* __restrict__ At, int rows, int cols,
-                                                       const double* __restrict__ in, int64_t ldin, int64_t V,
-                                                       double* __restrict__ out, float* __restrict__ out32,
-                                                       int64_t ldout) {
+template <class TIn>
+__global__ void __launch_bounds__(32 * kApplyWarps, 1)
+    k_apply_dmma(const double* __restrict__ At, int lda, int rows, int cols, int mt_chunk, const TIn* __restrict__ in,
+                 int64_t ldin, const int64_t* __restrict__ idx, int64_t V, double* __restrict__ out,
+                 float* __restrict__ out32, int64_t ldout, int rows_out, const double* add, double sign) {
   extern __shared__ __align__(16) double sA[];
-  const int MT = (rows + 7) / 8, KT = (cols + 3) / 4;
+  const int mt_first = blockIdx.y * mt_chunk;
+  const int MT = min(mt_chunk, (rows_out + 7) / 8 - mt_first), KT = (cols + 3) / 4;
   const int n_frag = MT * KT * 32;
   for (int i0 = threadIdx.x; i0 < n_frag; i0 += 8 * blockDim.x) {  // eight loads in flight per thread
     double vals[8];
@@ -324,8 +289,8 @@ __global__ void __launch_bounds__(256, 1) k_apply_dmma(const double* __restrict_
     for (int u = 0; u < 8; ++u) {
       const int i = i0 + u * blockDim.x;
       const int lane = i & 31, t = i >> 5, mt = t / KT, kt = t % KT;
-      const int r = 8 * mt + (lane >> 2), k = 4 * kt + (lane & 3);
-      vals[u] = (i < n_frag && r < rows && k < cols) ? At[static_cast<size_t>(k) * rows + r] : 0.0;
+      const int r = 8 * (mt_first + mt) + (lane >> 2), k = 4 * kt + (lane & 3);
+      vals[u] = (i < n_frag && r < rows && k < cols) ? __ldg(At + static_cast<size_t>(k) * lda + r) : 0.0;
     }
 #pragma unroll
     for (int u = 0; u < 8; ++u)
@@ -336,77 +301,54 @@ __global__ void __launch_bounds__(256, 1) k_apply_dmma(const double* __restrict_
   const int g = lane >> 2, q = lane & 3;
   const int64_t groups = (V + 7) / 8;
   const int64_t nwarps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
-  auto frag = [&](int64_t grp, int kt) -> double {  // this lane's B entry of k-step kt of a group
-    const int64_t vb = 8 * grp + g;
-    const int k = 4 * kt + q;
-    return (grp < groups && vb < V && k < cols) ? in[vb * ldin + k] : 0.0;
-  };
-  auto store = [&](int64_t v0, int mt0, const double (&d)[kApplyMtc][2]) {
+  for (int64_t grp = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + warp; grp < groups; grp += nwarps) {
+    // voxels past the last repeat its row (their outputs are not stored)
+    const int64_t vb = 8 * grp + g < V ? 8 * grp + g : V - 1;
+    const TIn* src = in + (idx ? idx[vb] : vb) * ldin + q;
+    auto frag = [&](int kt) -> TIn {  // this lane's B entry of k-step kt
+      return 4 * kt + q < cols ? __ldg(src + 4 * kt) : TIn(0);
+    };
+    for (int mt0 = 0; mt0 < MT; mt0 += kApplyMtc) {
+      const int nt = MT - mt0 < kApplyMtc ? MT - mt0 : kApplyMtc;
+      double d[kApplyMtc][2];
 #pragma unroll
-    for (int j = 0; j < kApplyMtc; ++j) {
-      const int r = 8 * (mt0 + j) + g;
-      if (mt0 + j >= MT || r >= rows) continue;
+      for (int j = 0; j < kApplyMtc; ++j) d[j][0] = d[j][1] = 0.0;
+      auto pass = [&](auto full) {
+        TIn bq[kApplyPf];
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int64_t vv = v0 + 2 * q + e;
-        if (vv < V) {
-          if (out) out[vv * ldout + r] = d[j][e];
-          if (out32) out32[vv * ldout + r] = static_cast<float>(d[j][e]);
-        }
-      }
-    }
-  };
-  int64_t grp = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + warp;
-  if constexpr (kRegs) {
-    double bn[kApplyKtr];
-#pragma unroll
-    for (int kt = 0; kt < kApplyKtr; ++kt) bn[kt] = kt < KT ? frag(grp, kt) : 0.0;
-    for (; grp < groups; grp += nwarps) {
-      double bc[kApplyKtr];
-#pragma unroll
-      for (int kt = 0; kt < kApplyKtr; ++kt) {
-        bc[kt] = bn[kt];
-        bn[kt] = kt < KT ? frag(grp + nwarps, kt) : 0.0;  // the next group's, in flight meanwhile
-      }
-      for (int mt0 = 0; mt0 < MT; mt0 += kApplyMtc) {
-        double d[kApplyMtc][2];
-#pragma unroll
-        for (int j = 0; j < kApplyMtc; ++j) d[j][0] = d[j][1] = 0.0;
-#pragma unroll
-        for (int kt = 0; kt < kApplyKtr; ++kt) {
-          if (kt >= KT) break;
-#pragma unroll
-          for (int j = 0; j < kApplyMtc; ++j)
-            if (mt0 + j < MT) dmma_m8n8k4(d[j][0], d[j][1], sA[((mt0 + j) * KT + kt) * 32 + lane], bc[kt]);
-        }
-        store(8 * grp, mt0, d);
-      }
-    }
-  } else {
-    for (; grp < groups; grp += nwarps) {
-      for (int mt0 = 0; mt0 < MT; mt0 += kApplyMtc) {
-        double d[kApplyMtc][2];
-#pragma unroll
-        for (int j = 0; j < kApplyMtc; ++j) d[j][0] = d[j][1] = 0.0;
-        // slot u holds k-step kt0 + u; once its DMMAs have read it, it is
-        // refilled with k-step kt0 + u + kApplyPf (no register moves, which
-        // would wait for loads still in flight)
-        double bq[kApplyPf];
-#pragma unroll
-        for (int u = 0; u < kApplyPf; ++u) bq[u] = frag(grp, u);
+        for (int u = 0; u < kApplyPf; ++u) bq[u] = frag(u);
+        const double* fa = sA + static_cast<size_t>(mt0) * KT * 32 + lane;
         for (int kt0 = 0; kt0 < KT; kt0 += kApplyPf) {
 #pragma unroll
           for (int u = 0; u < kApplyPf; ++u) {
             const int kt = kt0 + u;
             if (kt < KT) {
+              const double b = static_cast<double>(bq[u]);
 #pragma unroll
               for (int j = 0; j < kApplyMtc; ++j)
-                if (mt0 + j < MT) dmma_m8n8k4(d[j][0], d[j][1], sA[((mt0 + j) * KT + kt) * 32 + lane], bq[u]);
-              bq[u] = frag(grp, kt + kApplyPf);
+                if (decltype(full)::value || j < nt) dmma_m8n8k4(d[j][0], d[j][1], fa[(j * KT + kt) * 32], b);
+              bq[u] = frag(kt + kApplyPf);
             }
           }
         }
-        store(8 * grp, mt0, d);
+      };
+      if (nt == kApplyMtc)
+        pass(std::true_type{});
+      else
+        pass(std::false_type{});
+#pragma unroll
+      for (int j = 0; j < kApplyMtc; ++j) {
+        const int r = 8 * (mt_first + mt0 + j) + g;
+        if (j >= nt || r >= rows_out) continue;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int64_t vv = 8 * grp + 2 * q + e;
+          if (vv < V) {
+            const double o = add ? fma(sign, d[j][e], add[vv * ldout + r]) : d[j][e];
+            if (out) out[vv * ldout + r] = o;
+            if (out32) out32[vv * ldout + r] = static_cast<float>(o);
+          }
+        }
       }
     }
   }

@@ -272,6 +272,7 @@ struct csd_handle {
   // mtfrag), so an L2 fit is the single product c = P s; built with the factor
   DevBuf pfrag, ptmp;
   bool pfrag_valid = false;
+  DevBuf hmat;                // H itself (refinement of the solves)
   DevBuf hinv;                // H^{-1} of the current factor (L2 adjoint)
   bool hinv_valid = false;
   uint64_t hinv_key = 0;
@@ -529,6 +530,8 @@ void ensure_setup(csd_handle* h, const HostGtab& g, int radial_order, double zet
       const size_t csm = sizeof(double) * static_cast<size_t>(K) * K;
       CSD_CUDA(cudaFuncSetAttribute(csd::k_cholesky, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     static_cast<int>(csm)));
+      h->hmat.ensure(sizeof(double) * Kp * Kp);
+      CSD_CUDA(cudaMemcpyAsync(h->hmat.p, h->A.p, sizeof(double) * Kp * Kp, cudaMemcpyDeviceToDevice, st));
       csd::k_cholesky<<<1, 256, csm, st>>>(h->A.as<double>(), K, Kp, h->ok.as<int>());
       CSD_LAUNCH();
       int okv = 0;
@@ -854,16 +857,16 @@ bool sparse_fista(const csd_handle* h, int64_t n_work) {
 
 // One voxel per warp has the shorter iteration, two share the reads of G's
 // columns (per voxel-iteration 100 against 72 wavefronts at order 6): two
-// from about four times the voxels that one per warp holds at once (order 6:
-// 4,000 voxels 0.84 / 1.06 ms, 16,384 voxels 1.57 / 1.54 ms, 64,000 voxels
-// 4.07 / 3.77 ms; order 8: 8,000 voxels 1.56 / 1.80 ms, 16,000 voxels 2.43 /
-// 2.40 ms).  At order 4 one is faster at every size measured (64,000 voxels
+// from about seven times the voxels that one per warp holds at once (order 6:
+// 4,000 voxels 0.84 / 1.06 ms, 9,600 voxels 1.06 / 1.15 ms, 16,384 voxels 1.50 /
+// 1.53 ms, 64,000 voxels 4.18 / 3.80 ms; order 8: 8,000 voxels 1.56 / 1.80 ms,
+// 16,000 voxels 2.43 / 2.40 ms).  At order 4 one is faster at every size measured (64,000 voxels
 // 1.69 / 1.78 ms).
 void launch_fista_sparse(csd_handle* h, const csd::FistaParams& p) {
   switch (h->K) {
     case 29: launch_fista_sparse_p<29, 1, 16, 2>(h, p); break;
     case 72:
-      if (p.n_work > 64 * h->num_sms)
+      if (p.n_work > 112 * h->num_sms)
         launch_fista_sparse_p<72, 2, 16, 1>(h, p);
       else
         launch_fista_sparse_p<72, 1, 16, 1>(h, p);
@@ -1473,6 +1476,38 @@ void launch_fista(csd_handle* h, int MT, const csd::FistaParams& p) {
   }
 }
 
+// Whether one row tile of a matrix of `cols` columns fits in shared memory.
+bool apply_dmma_fits(const csd_handle* h, int cols) {
+  return sizeof(double) * 32 * static_cast<size_t>((cols + 3) / 4) <= static_cast<size_t>(h->smem_optin);
+}
+
+// out = A in per voxel on the FP64 tensor cores: A (rows x cols, transposed in
+// At with row stride lda), rows_out >= rows outputs (zeros past rows).
+template <class TIn>
+void launch_apply_dmma(csd_handle* h, const double* At, int lda, int rows, int cols, const TIn* in, int64_t ldin,
+                       const int64_t* idx, int64_t V, double* out, float* out32, int64_t ldout, int rows_out,
+                       const double* add = nullptr, double sign = 1.0) {
+  constexpr int W = csd::kApplyWarps;
+  const size_t tile = sizeof(double) * 32 * static_cast<size_t>((cols + 3) / 4);
+  const int MT = (rows_out + 7) / 8;
+  const int most = static_cast<int>(std::min<size_t>(MT, static_cast<size_t>(h->smem_optin) / tile));
+  // CTAs along the voxels: at least four groups of eight a warp where there are
+  // that many SMs; the row tiles split so that the grid fills them
+  const int64_t groups = (V + 7) / 8;
+  const int64_t bx_full = std::max<int64_t>(1, (groups + W - 1) / W);
+  int chunks = (MT + most - 1) / most;
+  chunks = static_cast<int>(std::max<int64_t>(chunks, std::min<int64_t>(MT, h->num_sms / std::min<int64_t>(bx_full, h->num_sms))));
+  const int mt_chunk = (MT + chunks - 1) / chunks;
+  chunks = (MT + mt_chunk - 1) / mt_chunk;
+  const int64_t bx = std::min<int64_t>(bx_full, std::max(1, h->num_sms / chunks));
+  const size_t smem = tile * mt_chunk;
+  auto* kern = csd::k_apply_dmma<TIn>;
+  CSD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  kern<<<dim3(static_cast<unsigned>(bx), static_cast<unsigned>(chunks)), 32 * W, smem, h->stream>>>(
+      At, lda, rows, cols, mt_chunk, in, ldin, idx, V, out, out32, ldout, rows_out, add, sign);
+  CSD_LAUNCH();
+}
+
 template <int KP>
 void launch_rhs_t(csd_handle* h, const float* d_data, int64_t V) {
   const size_t smem = sizeof(double) * (32 * KP + 64 * 33);
@@ -1496,13 +1531,18 @@ void launch_rhs_dmma_t(csd_handle* h, const float* d_data, int64_t V, float* sig
   CSD_LAUNCH();
 }
 
-// b = M^T s for every masked voxel into h->B; or, with `frag` / `out` set (the
-// packed Tikhonov operator, DMMA path only), c = P s into `out`.
-void launch_rhs(csd_handle* h, const float* d_data, int64_t V, float* sig_out = nullptr,
-                const double* frag = nullptr, double* out = nullptr) {
+// Whether c = P s with the Tikhonov operator serves an L2 fit of the table.
+bool l2_operator_ready(const csd_handle* h) { return h->dmma_rhs && h->pfrag_valid; }
+
+// b = M^T s for every masked voxel into h->B; or, with `l2_out` set, c = P s
+// (l2_operator_ready) into it.  A design that does not fit one CTA's shared
+// memory (radial order 8, or more than 288 samples) goes through the apply
+// kernel's chunks of row tiles, with the same sums: 32,000 voxels at order 8,
+// N = 259, 277 us on k_rhs's FMAs.
+void launch_rhs(csd_handle* h, const float* d_data, int64_t V, float* sig_out = nullptr, double* l2_out = nullptr) {
   if (h->dmma_rhs) {
-    const double* f = frag ? frag : h->mtfrag.as<double>();
-    double* o = out ? out : h->B.as<double>();
+    const double* f = l2_out ? h->pfrag.as<double>() : h->mtfrag.as<double>();
+    double* o = l2_out ? l2_out : h->B.as<double>();
     switch (h->Kp) {
       case 8: launch_rhs_dmma_t<8>(h, d_data, V, sig_out, f, o); return;
       case 32: launch_rhs_dmma_t<32>(h, d_data, V, sig_out, f, o); return;
@@ -1510,7 +1550,12 @@ void launch_rhs(csd_handle* h, const float* d_data, int64_t V, float* sig_out = 
       default: break;
     }
   }
-  if (frag) throw Error{CSD_ERR_INVALID, "the Tikhonov operator product needs the DMMA right-hand-side kernel"};
+  if (l2_out) throw Error{CSD_ERR_INVALID, "the Tikhonov operator product needs the DMMA right-hand-side kernel"};
+  if (apply_dmma_fits(h, h->N)) {
+    launch_apply_dmma<float>(h, h->M.as<double>(), h->K, h->K, h->N, d_data, h->N, h->vox.as<int64_t>(), V,
+                             h->B.as<double>(), nullptr, h->Kp, h->Kp);
+    return;
+  }
   switch (h->Kp) {
     case 8: launch_rhs_t<8>(h, d_data, V); break;
     case 32: launch_rhs_t<32>(h, d_data, V); break;
@@ -1538,6 +1583,27 @@ void launch_tikhonov(csd_handle* h, const double* B, double* X, int64_t V) {
     case 5: go(csd::k_tikhonov<5>); break;
     default: throw Error{CSD_ERR_INVALID, "Tikhonov kernel supports K <= 160"};
   }
+}
+
+void ensure_hinv(csd_handle* h);
+
+// H c = b for every voxel where the operator product does not apply (order 8,
+// long tables): the inverse's product with one step of refinement, c = H^-1 b,
+// c += H^-1 (b - H c), whose normal-equation residual is that of the
+// substitution (k_tikhonov: 2 K serial steps a voxel, each a division and a
+// shuffle).  Measured at 3,001 voxels, order 8: 355 -> 65 us; relative error
+// against a 64-bit solve over orders 6 and 8, 150-515 samples, lambda 1e-8 to
+// 0.05: see the bounds in the differentiable fit's tests.
+void solve_l2(csd_handle* h, const double* B, double* X, int64_t V) {
+  if (V <= 0) return;
+  ensure_hinv(h);
+  const int K = h->K, Kp = h->Kp;
+  h->adjW.ensure(sizeof(double) * static_cast<size_t>(V) * Kp);
+  double* R = h->adjW.as<double>();
+  const double *Hi = h->hinv.as<double>(), *H = h->hmat.as<double>();
+  launch_apply_dmma<double>(h, Hi, K, K, K, B, Kp, nullptr, V, X, nullptr, Kp, Kp);
+  launch_apply_dmma<double>(h, H, Kp, K, K, X, Kp, nullptr, V, R, nullptr, Kp, Kp, B, -1.0);
+  launch_apply_dmma<double>(h, Hi, K, K, K, R, Kp, nullptr, V, X, nullptr, Kp, Kp, X, 1.0);
 }
 
 void launch_epilogue_ffma(csd_handle* h, const csd::EpilogueParams& p) {
@@ -1930,17 +1996,16 @@ FitInfo run_fit(csd_handle* h, const float* d_data, const uint8_t* d_mask, int64
   CSD_CUDA(cudaMemsetAsync(h->itotal.p, 0, 3 * sizeof(unsigned long long), st));
 
   // Tikhonov with the DMMA product: c = P s directly into X (no b)
-  const bool l2_operator = spec->regularization == CSD_REG_L2 && h->dmma_rhs && h->pfrag_valid;
-  const double* rhs_frag = l2_operator ? h->pfrag.as<double>() : nullptr;
+  const bool l2_operator = spec->regularization == CSD_REG_L2 && l2_operator_ready(h);
   double* rhs_out = l2_operator ? h->X.as<double>() : nullptr;
   if (data_on_host) {
     // `d_data` aliases pinned host memory: read each masked row once over the
     // bus and keep a compact device copy for every later pass.
     h->sig.ensure(sizeof(float) * static_cast<size_t>(V) * N);
-    launch_rhs(h, d_data, V, h->sig.as<float>(), rhs_frag, rhs_out);
+    launch_rhs(h, d_data, V, h->sig.as<float>(), rhs_out);
     h->sig_compact = h->sig.as<float>();
   } else {
-    launch_rhs(h, d_data, V, nullptr, rhs_frag, rhs_out);
+    launch_rhs(h, d_data, V, nullptr, rhs_out);
   }
   record(h, 2);
 
@@ -2021,7 +2086,7 @@ FitInfo run_fit(csd_handle* h, const float* d_data, const uint8_t* d_mask, int64
   } else if (spec->regularization == CSD_REG_L2) {
     kind = 2;
     record(h, 6);
-    if (!l2_operator) launch_tikhonov(h, h->B.as<double>(), h->X.as<double>(), V);
+    if (!l2_operator) solve_l2(h, h->B.as<double>(), h->X.as<double>(), V);
     record(h, 7);
     it_final = nullptr;
     CSD_CUDA(cudaMemsetAsync(h->conv.p, 1, V, st));
@@ -2071,10 +2136,10 @@ FitInfo run_fit(csd_handle* h, const float* d_data, const uint8_t* d_mask, int64
           // Tikhonov reference RSS per voxel (src/fit.rs:436-438).
           h->Xl2.ensure(sizeof(double) * V * Kp);
           h->rss_l2.ensure(sizeof(double) * V);
-          if (h->dmma_rhs && h->pfrag_valid && !data_on_host)  // one product, as the L2 fit
-            launch_rhs(h, d_data, V, nullptr, h->pfrag.as<double>(), h->Xl2.as<double>());
+          if (l2_operator_ready(h) && !data_on_host)  // one product, as the L2 fit
+            launch_rhs(h, d_data, V, nullptr, h->Xl2.as<double>());
           else
-            launch_tikhonov(h, h->B.as<double>(), h->Xl2.as<double>(), V);
+            solve_l2(h, h->B.as<double>(), h->Xl2.as<double>(), V);
           csd::EpilogueParams rp = ep;
           rp.X = h->Xl2.as<double>();
           rp.scatter = false;
@@ -2732,7 +2797,7 @@ void csd_destroy(csd_handle* h) {
                     &h->pbest, &h->psel, &h->pact, &h->palpha_sel, &h->pit_sel, &h->pconv_sel,
                     &h->palpha_fb, &h->pit_fb, &h->pconv_fb, &h->pcode, &h->gdig, &h->gfexp, &h->flagged,
                     &h->mixstat, &h->pcoef, &h->pmat, &h->pout, &h->pgt, &h->pgv, &h->pdir, &h->pconst,
-                    &h->iota, &h->adjW, &h->adjovf, &h->adjstat, &h->adjconst, &h->hinv,
+                    &h->iota, &h->adjW, &h->adjovf, &h->adjstat, &h->adjconst, &h->hinv, &h->hmat,
                     &h->gdtab, &h->gdq, &h->tuneB, &h->tuneX, &h->tuneIt, &h->tuneConv, &h->tuneQ,
                     &h->schedY, &h->schedPend, &h->schedKey, &h->schedOrder, &h->schedCnt,
                     &h->schedD, &h->schedU, &h->schedN, &h->ppark, &h->gtf32, &h->x32, &h->kktv, &h->kktovf,

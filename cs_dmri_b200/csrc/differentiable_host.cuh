@@ -40,9 +40,8 @@ void run_fit_batch(csd_handle* h, const float* d_sig, int64_t V, const HostGtab&
   csd::k_iota<<<grid1(V), 256, 0, st>>>(h->vox.as<int64_t>(), V);
   CSD_LAUNCH();
   // Tikhonov with the DMMA product c = P s, as the volume fit does
-  const bool l2_operator = !is_l1 && h->dmma_rhs && h->pfrag_valid;
-  launch_rhs(h, d_sig, V, nullptr, l2_operator ? h->pfrag.as<double>() : nullptr,
-             l2_operator ? h->X.as<double>() : nullptr);
+  const bool l2_operator = !is_l1 && l2_operator_ready(h);
+  launch_rhs(h, d_sig, V, nullptr, l2_operator ? h->X.as<double>() : nullptr);
   if (is_l1) {
     ensure_mom(h, spec->max_iter);
     if (d_warm) {
@@ -78,7 +77,7 @@ void run_fit_batch(csd_handle* h, const float* d_sig, int64_t V, const HostGtab&
     if (d_iters)
       CSD_CUDA(cudaMemcpyAsync(d_iters, h->iters.p, sizeof(uint32_t) * V, cudaMemcpyDeviceToDevice, st));
   } else {
-    if (!l2_operator) launch_tikhonov(h, h->B.as<double>(), h->X.as<double>(), V);
+    if (!l2_operator) solve_l2(h, h->B.as<double>(), h->X.as<double>(), V);
     if (d_iters) {
       csd::k_fill_u32<<<grid1(V), 256, 0, st>>>(d_iters, V, 1u);
       CSD_LAUNCH();
@@ -191,36 +190,8 @@ struct L2Adj {
 
 void launch_apply64(csd_handle* h, const double* At, int rows, int cols, const double* in, int64_t ldin, int64_t V,
                     double* out, float* out32, int64_t ldout) {
-  // tensor-core path when the matrix fits in one CTA's shared memory
-  const size_t dmma_smem = sizeof(double) * 32 * static_cast<size_t>((rows + 7) / 8) * ((cols + 3) / 4);
-  if (dmma_smem <= static_cast<size_t>(h->smem_optin)) {
-    const int64_t groups = (V + 7) / 8;
-    const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((groups + 7) / 8, h->num_sms));
-    auto go = [&](auto kern) {
-      CSD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(dmma_smem)));
-      kern<<<static_cast<unsigned>(blocks), 256, dmma_smem, h->stream>>>(At, rows, cols, in, ldin, V, out, out32,
-                                                                         ldout);
-      CSD_LAUNCH();
-    };
-    if ((cols + 3) / 4 <= csd::kApplyKtr)
-      go(csd::k_apply_dmma<true>);
-    else
-      go(csd::k_apply_dmma<false>);
-    return;
-  }
-  const size_t per_warp = sizeof(double) * 8 * static_cast<size_t>(cols);
-  const int warps = static_cast<int>(std::max<size_t>(1, std::min<size_t>(8, (100u << 10) / per_warp)));
-  const size_t smem = per_warp * warps;
-  if (smem > static_cast<size_t>(h->smem_optin)) throw Error{CSD_ERR_INVALID, "matrix too wide to apply"};
-  CSD_CUDA(cudaFuncSetAttribute(csd::k_apply64, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  int per_sm = 0;
-  CSD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, csd::k_apply64, 32 * warps, smem));
-  const int64_t groups = (V + 7) / 8;
-  const int64_t blocks = std::max<int64_t>(
-      1, std::min<int64_t>((groups + warps - 1) / warps, static_cast<int64_t>(h->num_sms) * std::max(per_sm, 1)));
-  csd::k_apply64<<<static_cast<unsigned>(blocks), 32 * warps, smem, h->stream>>>(At, rows, cols, in, ldin, V, out,
-                                                                                 out32, ldout);
-  CSD_LAUNCH();
+  if (!apply_dmma_fits(h, cols)) throw Error{CSD_ERR_INVALID, "matrix too wide to apply"};
+  launch_apply_dmma<double>(h, At, rows, rows, cols, in, ldin, nullptr, V, out, out32, ldout, rows);
 }
 
 // RTOP constants for (radial_order, zeta), built once and kept on the handle.
