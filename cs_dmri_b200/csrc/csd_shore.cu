@@ -736,13 +736,36 @@ void ensure_sched(csd_handle* h, int64_t V) {
 // One FISTA launch, or the two-pass schedule: pass 1 to the cap, the parked
 // voxels ordered, pass 2 resuming them.  go(params) launches the kernel, whose
 // grid holds `slots` voxels at a time.
+void launch_fista_sparse(csd_handle* h, const csd::FistaParams& p);
+
+// From one to kHybridWaves waves of DMMA slots the second pass runs on the
+// sparse kernel: 80 iterations at the DMMA warps' throughput (most voxels of a
+// large alpha end there), then the slowest voxels first on warps that take a
+// sixth of the time an iteration.  Per volume fit, N = 259, against a single
+// DMMA pass and the two passes both on DMMA slots:
+//   order 6, alpha 0.01:  38,760 voxels 2.42 ms (single 3.22), 77,520 voxels
+//     4.35 (two DMMA passes 5.27), 124,032 voxels 5.81 (6.34), 193,800 voxels
+//     8.77 (8.64), 299,432 voxels 13.4 (12.6)
+//   order 6, alpha 0.05:  38,760 voxels 0.44 ms (sparse alone 0.47), 65,892
+//     voxels 0.57 (0.63)
+//   order 4, alpha 0.01:  38,760 voxels 1.09 ms (1.33), 124,032 voxels 2.15
+//     (2.42), 310,080 voxels 4.86 (4.65)
+constexpr int64_t kHybridWaves = 8;
+
+bool hybrid_fista(const csd_handle* h, const csd::FistaParams& p, int64_t slots) {
+  const int cap = sched_cap(h);
+  return (h->K == 29 || h->K == 72) && h->opt_shape == 0 && cap > 0 && h->sched_off == 0 && p.cap == 0 &&
+         !p.n_work_dev && p.max_iter > 2 * cap && p.n_work >= slots && p.n_work < kHybridWaves * slots;
+}
+
 template <class Go>
 void launch_fista_sched(csd_handle* h, const csd::FistaParams& p, int64_t slots, Go go) {
+  const bool hybrid = hybrid_fista(h, p, slots);
   csd::FistaParams q = p;
   q.gfrag = h->gfrag.as<double>();
   q.mom = h->mom.as<double>();
   cudaStream_t st = h->stream;
-  if (!sched_enabled(h, p, slots)) {
+  if (!hybrid && !sched_enabled(h, p, slots)) {
     go(q);
     return;
   }
@@ -767,9 +790,8 @@ void launch_fista_sched(csd_handle* h, const csd::FistaParams& p, int64_t slots,
   go(q1);
   csd::k_sched_hist<<<h->num_sms, 256, 0, st>>>(key, n_pend, hist, p.iter_total ? p.iter_total + 2 : nullptr);
   CSD_LAUNCH();
-  csd::k_sched_order<<<h->num_sms, csd::kSchedBins, 0, st>>>(pend, key, n_pend, hist, cursor, order);
+  csd::k_sched_order<<<h->num_sms, csd::kSchedBins, 0, st>>>(pend, key, n_pend, hist, cursor, order, p.queue);
   CSD_LAUNCH();
-  CSD_CUDA(cudaMemsetAsync(p.queue, 0, sizeof(unsigned long long), st));
   csd::FistaParams q2 = q1;
   q2.resume = 1;
   q2.warm = nullptr;
@@ -777,7 +799,10 @@ void launch_fista_sched(csd_handle* h, const csd::FistaParams& p, int64_t slots,
   q2.n_work_dev = n_pend;
   q2.pend = nullptr;
   q2.pend_key = nullptr;
-  go(q2);
+  if (hybrid)
+    launch_fista_sparse(h, q2);
+  else
+    go(q2);
 }
 
 template <int MT, int WARPS, bool NONNEG>
@@ -836,23 +861,28 @@ void launch_fista_sparse_p(csd_handle* h, const csd::FistaParams& p) {
     launch_fista_sparse_t<K, P, MAXWARPS, MINCTAS, false>(h, p);
 }
 
-// Whether a fit of n_work voxels takes the sparse kernel (handle option
+// Whether a fit of n_work voxels takes the sparse kernel alone (handle option
 // CSD_OPT_FISTA_SHAPE left at 0; every kernel computes the same iterates).
-// Measured per volume fit on B200, sparse against k_fista_v3, N = 259:
-//   order 4:   74,088 voxels 1.85 / 1.94 ms, 300,763 voxels 6.41 / 5.25 ms
-//   order 6:    4,000 voxels 0.84 / 2.80 ms, 74,088 voxels 4.29 / 4.32 ms,
-//             125,000 voxels 6.97 / 6.25 ms
-//   order 8:   32,000 voxels 4.56 / 6.87 ms, 300,763 voxels 33.2 / 47.5 ms
+// Measured per volume fit on B200, sparse against k_fista_v3, N = 259, alpha
+// 0.01:
+//   order 4:  15,504 voxels 0.68 / 1.33 ms, 300,763 voxels 6.41 / 5.25 ms
+//   order 6:   4,000 voxels 0.84 / 2.80 ms, 15,504 voxels 1.26 / 2.38 ms,
+//            125,000 voxels 6.97 / 6.25 ms
+//   order 8:  32,000 voxels 4.56 / 6.87 ms, 300,763 voxels 33.2 / 47.5 ms
 // A warp of k_fista_v3 takes 2 us an iteration for its eight voxels and the
 // slowest voxel's up to 1,000 iterations set a small fit's time; a sparse warp
-// takes 0.3 us.  From four waves of slots the DMMA kernel's two-pass schedule
-// hides that tail and its throughput decides - except at order 8, where G's
-// tiles do not fit in shared memory beside the slots' vectors and 9 % of y's
-// entries are non-zero.
+// takes 0.3 us.  From one wave of DMMA slots the first iterations of a fit are
+// bound by throughput, where the DMMA slots are ahead (alpha 0.05, 19
+// iterations, 65,892 voxels: 0.63 / 0.57 ms at order 6, 0.41 / 0.38 at order
+// 4), and hybrid_fista takes over; with the schedule off (a walk that launches
+// point by point) sparse warps up to four waves.  At order 8 G's tiles do not
+// fit in shared memory beside the slots' vectors and 9 % of y's entries are
+// non-zero: always sparse.
 bool sparse_fista(const csd_handle* h, int64_t n_work) {
   if (h->K == 145) return true;
   if (h->opt_shape != 0 || (h->K != 29 && h->K != 72)) return false;
-  return n_work < kSchedMinWaves * h->num_sms * 16 * 8;
+  const int64_t slots = static_cast<int64_t>(h->num_sms) * 16 * 8;
+  return n_work < (h->sched_off > 0 ? kSchedMinWaves : 1) * slots;
 }
 
 // One voxel per warp has the shorter iteration, two share the reads of G's
@@ -1077,9 +1107,8 @@ void launch_fista_mixed(csd_handle* h, const csd::FistaParams& p) {
     CSD_LAUNCH();
     csd::k_sched_hist<<<h->num_sms, 256, 0, st>>>(key, n_pend, hist, p.iter_total ? p.iter_total + 2 : nullptr);
     CSD_LAUNCH();
-    csd::k_sched_order<<<h->num_sms, csd::kSchedBins, 0, st>>>(pend, key, n_pend, hist, cursor, order);
+    csd::k_sched_order<<<h->num_sms, csd::kSchedBins, 0, st>>>(pend, key, n_pend, hist, cursor, order, p.queue);
     CSD_LAUNCH();
-    CSD_CUDA(cudaMemsetAsync(p.queue, 0, sizeof(unsigned long long), st));
     csd::MixedParams q2 = q1;
     q2.resume = 1;
     q2.warm = nullptr;

@@ -432,7 +432,20 @@ __device__ __forceinline__ unsigned dmma_fista_step(const double* sG, double* yb
 #pragma unroll
   for (int mt = 0; mt < MT; ++mt) acc[mt][0] = acc[mt][1] = 0.0;
   // A k-step whose four y entries are exactly zero for all eight voxels adds
-  // only zeros (soft thresholding keeps most of y at 0): only the live ones run.
+  // only zeros (soft thresholding keeps most of y at 0): only the live ones run
+  // (the few k-steps of small orders unrolled, their fragments loaded ahead).
+  if constexpr (MT <= 4) {
+    ksteps = __popc(live[0] & ((1u << KT) - 1u));
+    double bf[KT];
+#pragma unroll
+    for (int kt = 0; kt < KT; ++kt) bf[kt] = ybuf[(4 * kt + q) * 8 + g];
+#pragma unroll
+    for (int kt = 0; kt < KT; ++kt) {
+      if (!((live[0] >> kt) & 1u)) continue;
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt) dmma_m8n8k4(acc[mt][0], acc[mt][1], sG[(mt * KT + kt) * 32 + lane], bf[kt]);
+    }
+  } else
 #pragma unroll
   for (int w = 0; w < LW; ++w) {
     unsigned m = live[w] & (KT - 32 * w >= 32 ? kFull : (1u << (KT - 32 * w)) - 1u);
@@ -675,6 +688,7 @@ __global__ void __launch_bounds__(256) k_sched_hist(const float* __restrict__ ke
                                                     unsigned* __restrict__ hist,
                                                     unsigned long long* __restrict__ parked_total) {
   __shared__ unsigned sh[kSchedBins];
+  if (*n_key == 0) return;
   if (parked_total && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(parked_total, *n_key);
   for (int b = threadIdx.x; b < kSchedBins; b += blockDim.x) sh[b] = 0;
   __syncthreads();
@@ -690,12 +704,16 @@ __global__ void __launch_bounds__(256) k_sched_hist(const float* __restrict__ ke
 // order[] = pend[] by bucket, highest bucket first.  Block `blk` handles one
 // contiguous segment: it reserves a run in each bucket with one atomic per
 // bucket (cursor zeroed by the caller), then places its entries.  256 threads.
+// The work queue is reset for the pass that follows.
 __global__ void __launch_bounds__(256) k_sched_order(const int64_t* __restrict__ pend, const float* __restrict__ key,
                                                      const unsigned long long* __restrict__ n_key,
                                                      const unsigned* __restrict__ hist, unsigned* __restrict__ cursor,
-                                                     int64_t* __restrict__ order) {
+                                                     int64_t* __restrict__ order,
+                                                     unsigned long long* __restrict__ queue) {
   __shared__ unsigned scan[kSchedBins], base[kSchedBins], cnt[kSchedBins];
   const int t = threadIdx.x;
+  if (blockIdx.x == 0 && t == 0) *queue = 0;
+  if (*n_key == 0) return;
   // base[b] = entries in buckets above b (inclusive scan over reversed buckets)
   scan[t] = hist[kSchedBins - 1 - t];
   cnt[t] = 0;

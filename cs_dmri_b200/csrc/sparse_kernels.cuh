@@ -288,10 +288,11 @@ __global__ void __launch_bounds__(32 * MAXWARPS, MINCTAS) k_fista_sparse(FistaPa
   using S = SparseShape<K, P>;
   constexpr bool WIDE = P == 1 && K == 72;
   extern __shared__ __align__(16) unsigned char sp_smem[];
+  const unsigned long long n_work = p.n_work_dev ? *p.n_work_dev : static_cast<unsigned long long>(p.n_work);
+  if (n_work == 0) return;
   SparseFista<K, P, NONNEG, WIDE> f;
   f.init(p.G, sp_smem);
   __syncthreads();
-  const unsigned long long n_work = p.n_work_dev ? *p.n_work_dev : static_cast<unsigned long long>(p.n_work);
   const int it0 = p.resume ? p.cap : 0;
   const double c = p.step * p.n_inv;
   unsigned long long executed = 0;

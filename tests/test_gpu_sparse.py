@@ -32,11 +32,14 @@ def fit(ph, data, mask, **kw):
 
 
 @pytest.mark.parametrize("order", [4, 6])
-@pytest.mark.parametrize("v", [1, 33, 601, 9475, 9999])  # order 6: two voxels per warp from 9,473
+@pytest.mark.parametrize("v", [1, 33, 601, 16577, 18943, 18944, 19001])
 @pytest.mark.parametrize("kw", [dict(alpha_mode="fixed", alpha=0.01),
                                 dict(alpha_mode="fixed", alpha=0.02, non_negative=True, max_iter=37),
                                 dict(alpha_mode="alpha-ratio", alpha_ratio=0.01)])
 def test_matches_the_dmma_kernel_bit_for_bit(order, v, kw):
+    """Order 6: two voxels per warp from 16,577; from 18,944 (one wave of DMMA
+    slots) the first 80 iterations run on those and the rest on sparse warps.
+    """
     from cs_dmri_b200 import _abi
     ph, data, mask = tiled(v)
     sparse = fit(ph, data, mask, radial_order=order, **kw)
