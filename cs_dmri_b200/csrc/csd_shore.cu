@@ -601,10 +601,10 @@ void ensure_icls_setup(csd_handle* h, int radial_order, double zeta, double eps)
   csd::k_icls_w<<<(m_pad + 127) / 128, 128, 0, st>>>(h->Le.as<double>(), K, Kp, h->Cmat.as<double>(), m, m_pad,
                                                       h->Wi.as<double>());
   CSD_LAUNCH();
-  // the Gram form: active sets one entry per lane (nsh <= 32), 11 constraint
+  // the Gram form: active sets one entry per lane (nsh <= 28), 11 constraint
   // slots per lane (m_pad = 352), x~ in <= 3 registers per lane
   h->icls_nsh = h->icls_qmax;
-  h->icls_gram = h->icls_nsh <= 32 && m_pad == 32 * kIclsGramCpl && Kp <= 96 &&
+  h->icls_gram = h->icls_nsh <= csd::kIclsGramQ && m_pad == 32 * kIclsGramCpl && Kp <= 96 &&
                  csd::icls_gram_smem(h->icls_nsh, m_pad) <= static_cast<size_t>(h->smem_optin);
   if (h->icls_gram) {
     const int64_t n_gam = static_cast<int64_t>(m_pad) * m_pad;
@@ -1744,8 +1744,8 @@ void launch_icls_t(csd_handle* h, csd::IclsParams p) {
 template <int RPL>
 void launch_icls_gram_t(csd_handle* h, const csd::IclsParams& p) {
   csd::IclsGramParams g{};
-  g.B = p.B;
-  g.Ginv = h->icls_ginv.as<double>();
+  launch_apply_dmma<double>(h, h->icls_ginv.as<double>(), p.Kp, p.K, p.K, p.B, p.Kp, nullptr, p.V, p.X, nullptr, p.Kp,
+                            p.Kp);
   g.Gam = h->icls_gam.as<double>();
   g.UT = h->icls_ut.as<double>();
   g.Y = h->icls_y.as<double>();

@@ -478,16 +478,16 @@ __global__ void __launch_bounds__(32 * kIclsWarps) k_icls(IclsParams p) {
 //   v = w_p - W_A r,  so the constraint values s = W^T x~ move by
 //   t (Gamma[:, p] - Gamma[:, A] r) and x = L^-T x~ by t (u_p - U_A r),
 //   U = L^-T W = G^-1 C^T (once per table).
-// A step therefore costs (q + 1) columns of Gamma and of U^T instead of the
-// K-wide products with Q1, and the scan for the most violated constraint
+// A constraint that joins therefore costs (q + 1) columns of Gamma instead of
+// K-wide products with Q1 at every step, and the scan for the most violated constraint
 // reads s from registers instead of recomputing W^T x~ (m x K) every
 // iteration.  The unconstrained minimiser x0 = G^-1 b is one product with
-// the inverse (no per-voxel substitution), and the first s = C x0 comes from
+// the inverse over all voxels (no per-voxel substitution), and the first s = C x0 comes from
 // C = Y P: z0 = P x0 (one term per column) and s = Y z0, with Y (nsh x m) in
 // shared memory.  The reference's multiplier rule is kept as is (a full step
 // pushes t for the new constraint), so drops follow its iteration path; the
 // carried s and x differ from recomputed ones by rounding only.  Active sets
-// of up to 32 are held one entry per lane (rank C = nsh <= 28 for lmax <= 6).
+// of up to 28 are held one entry per lane (rank C = nsh <= 28 for lmax <= 6).
 
 __global__ void k_icls_gram_setup(const double* __restrict__ W, int K, int m_pad, double* __restrict__ Gam) {
   const int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -529,14 +529,12 @@ __global__ void k_icls_gram_solves(const double* __restrict__ L, int K, int Kp, 
 }
 
 struct IclsGramParams {
-  const double* B;      // V x Kp: M^T s
-  const double* Ginv;   // Kp x Kp: (M^T M + eps I)^-1, symmetric
   const double* Gam;    // m_pad x m_pad: W^T W
   const double* UT;     // m_pad x Kp: row c = u_c = L^-T w_c = G^-1 c_c
   const double* Y;      // nsh x m_pad: C = Y P
   const double* pf;     // K: the non-zero of column col of P ...
   const int* jcol;      // K: ... and its row
-  double* X;            // V x Kp out
+  double* X;            // V x Kp: x0 = G^-1 M^T s in, x out
   uint32_t* iters;      // V
   uint8_t* conv;        // V
   int64_t V;
@@ -547,31 +545,108 @@ struct IclsGramParams {
   unsigned long long* iter_total;
 };
 
-constexpr int kIclsGramWarps = 16;
-constexpr int kIclsGramRs = 33;                     // row stride of R (conflict-free rows and columns)
-// Per warp: R (32 x 33); at the start of a voxel, before R is in use, its
-// first K entries hold x0 and entries 1024.. hold z0.
+constexpr int kIclsGramWarps = 20;
+constexpr int kIclsGramQ = 28;                      // largest active set (rank C at lmax 6)
+constexpr int kIclsGramRs = kIclsGramQ + 1;         // row stride of R (odd: conflict-free rows and columns)
+// Per warp: R, with a row for every lane (rows past the active set are read
+// and not used); at the start of a voxel, before R is in use, its first K
+// entries hold x0 and entries 96.. hold z0.
 constexpr int kIclsGramWarpDoubles = 32 * kIclsGramRs;
 
 __host__ __device__ inline size_t icls_gram_smem(int nsh, int m_pad) {
   return sizeof(double) * (static_cast<size_t>(nsh) * m_pad + static_cast<size_t>(kIclsGramWarps) * kIclsGramWarpDoubles);
 }
 
+// a / d by the correctly rounded reciprocal rd = 1 / d: the product corrected
+// once by its exact remainder (Markstein, IBM J. Res. Dev. 34(1), 1990), the
+// rounded quotient for operands away from the range's ends.
+__device__ __forceinline__ double quotient(double a, double d, double rd) {
+  const double q0 = __dmul_rn(a, rd);
+  return fma(fma(-d, q0, a), rd, q0);
+}
+
+// The lane of the smallest value among the lanes that have one, the lowest
+// lane on ties (-1: none): by the order-preserving bits of the value, high
+// word first.
+__device__ __forceinline__ int warp_argmin(double v, bool has) {
+  const long long b = __double_as_longlong(v + 0.0);  // -0 as 0
+  const unsigned long long key =
+      static_cast<unsigned long long>(b) ^ (b < 0 ? 0xffffffffffffffffull : 0x8000000000000000ull);
+  const unsigned hi = static_cast<unsigned>(key >> 32), lo = static_cast<unsigned>(key);
+  const unsigned mh = __reduce_min_sync(kFull, has ? hi : 0xffffffffu);
+  const bool in = has && hi == mh;
+  const unsigned ml = __reduce_min_sync(kFull, in ? lo : 0xffffffffu);
+  return __ffs(__ballot_sync(kFull, in && lo == ml)) - 1;
+}
+
+// s (constraint lane + 32 c) += sum over entries i < q of coef_i Gamma[:, a_i].
+template <int CPL>
+__device__ __forceinline__ void icls_gram_move(double (&s)[CPL], const double* __restrict__ Gam, int mp, int lane, int q,
+                                               double coef, int a) {
+#pragma unroll 1
+  for (int i = 0; i < q; ++i) {
+    const double ci = __shfl_sync(kFull, coef, i);
+    const double* g = Gam + static_cast<size_t>(__shfl_sync(kFull, a, i)) * mp + lane;
+    double col[CPL];
+#pragma unroll
+    for (int c = 0; c < CPL; ++c) col[c] = __ldg(g + 32 * c);
+#pragma unroll
+    for (int c = 0; c < CPL; ++c) s[c] = fma(ci, col[c], s[c]);
+  }
+}
+
+// x (row lane + 32 c) += coef u_a.
+template <int RPL>
+__device__ __forceinline__ void icls_gram_x(double (&xt)[RPL], const double* __restrict__ UT, int Kp, int lane, double coef,
+                                            int a) {
+  const double* w = UT + static_cast<size_t>(a) * Kp + lane;
+#pragma unroll
+  for (int c = 0; c < RPL; ++c)
+    if (lane + 32 * c < Kp) xt[c] = fma(coef, __ldg(w + 32 * c), xt[c]);
+}
+
 // One warp per voxel, voxels from an atomic queue.  Constraint c lives on
 // lane c % 32 (slot c / 32): its value s and active flag in registers; entry
-// i < q of the active set (its constraint, multiplier, d1, r) on lane i.
+// i < q <= 28 of the active set (its constraint, multiplier, d1, r) on lane i.
+// A step only records what it adds to the coefficient of each active
+// constraint: s moves once per constraint that joins (the scan is its only
+// reader), by one column of Gamma per entry and one per dropped constraint,
+// and x once per constraint that leaves or is active at the end.  Bound by a
+// warp's chain of dependent steps (16 steps a voxel over 4.6 active
+// constraints, order 6, 64,000 voxels): before, 250,000 cycles a voxel, of
+// them 88,000 in the moves of s and x at every step (latency of the L2 reads),
+// 59,000 in the substitutions (a division per entry on the chain, now a
+// corrected product with the diagonal's reciprocal), 17,000 in x0 (now one
+// tensor-core product over all voxels).  One column of Gamma in flight keeps a
+// thread at 96 registers, so 20 warps fit an SM: 1.68 ms a fit against 1.80
+// with two columns and 16 warps, and 3.05 before.
 template <int RPL, int CPL>  // ceil(K / 32); m_pad / 32
 __global__ void __launch_bounds__(32 * kIclsGramWarps, 1) k_icls_gram(IclsGramParams p) {
   extern __shared__ __align__(16) double gsm[];
   const int K = p.K, Kp = p.Kp, m = p.m, mp = p.m_pad, nsh = p.nsh;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double* Ysh = gsm;  // [nsh][m_pad]
+  __shared__ unsigned short zcol[96], zstart[33];  // the columns of P that feed each z0 entry, in index order
   for (int e = threadIdx.x; e < nsh * mp; e += blockDim.x) Ysh[e] = p.Y[e];
+  if (warp == 0) {
+    int n = 0;
+    for (int col = 0; col < K; ++col) n += p.jcol[col] == lane;
+    int end = n;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int up = __shfl_up_sync(kFull, end, o);
+      if (lane >= o) end += up;
+    }
+    zstart[lane + 1] = static_cast<unsigned short>(end);
+    if (lane == 0) zstart[0] = 0;
+    int at = end - n;
+    for (int col = 0; col < K; ++col)
+      if (p.jcol[col] == lane) zcol[at++] = static_cast<unsigned short>(col);
+  }
   __syncthreads();
   double* R = gsm + static_cast<size_t>(nsh) * mp + static_cast<size_t>(warp) * kIclsGramWarpDoubles;
-  double* x0s = R;          // [K], K <= 1024
-  double* z0 = R + 1024;    // [32]
-  const int qcap = nsh < 32 ? nsh : 32;
+  double* x0s = R;          // [K], K <= 96
+  double* z0 = R + 96;      // [32]
+  const int qcap = nsh < kIclsGramQ ? nsh : kIclsGramQ;
   unsigned long long executed = 0;
 
   while (true) {
@@ -581,32 +656,22 @@ __global__ void __launch_bounds__(32 * kIclsGramWarps, 1) k_icls_gram(IclsGramPa
     if (vq >= static_cast<unsigned long long>(p.V)) break;
     const int64_t v = static_cast<int64_t>(vq);
 
-    // x0 = G^-1 M^T s (icls.rs:271-273) as one product with the inverse
-    // (b staged in the warp's slice, G^-1 read by rows: coalesced over lanes)
-    for (int k = lane; k < K; k += 32) x0s[k] = p.B[v * Kp + k];
-    __syncwarp();
+    // x0 = G^-1 M^T s (icls.rs:271-273), left in X by the product over all voxels
     double xt[RPL];  // the iterate x, row lane + 32 c
-#pragma unroll
-    for (int c = 0; c < RPL; ++c) xt[c] = 0.0;
-    for (int k = 0; k < K; ++k) {
-      const double bk = x0s[k];
-      const double* gk = p.Ginv + static_cast<size_t>(k) * Kp + lane;
-#pragma unroll
-      for (int c = 0; c < RPL; ++c)
-        if (lane + 32 * c < K) xt[c] = fma(__ldg(gk + 32 * c), bk, xt[c]);
-    }
-    __syncwarp();
-    // s = C x0 = Y (P x0): z0[j] sums its columns in index order
 #pragma unroll
     for (int c = 0; c < RPL; ++c) {
       const int row = lane + 32 * c;
+      xt[c] = row < K ? p.X[v * Kp + row] : 0.0;
       if (row < K) x0s[row] = xt[c];
     }
+    // s = C x0 = Y (P x0): z0[j] sums its columns in index order
     __syncwarp();
     if (lane < nsh) {
       double zj = 0.0;
-      for (int col = 0; col < K; ++col)
-        if (__ldg(p.jcol + col) == lane) zj = fma(__ldg(p.pf + col), x0s[col], zj);
+      for (int e = zstart[lane]; e < zstart[lane + 1]; ++e) {
+        const int col = zcol[e];
+        zj = fma(__ldg(p.pf + col), x0s[col], zj);
+      }
       z0[lane] = zj;
     }
     __syncwarp();
@@ -623,6 +688,8 @@ __global__ void __launch_bounds__(32 * kIclsGramWarps, 1) k_icls_gram(IclsGramPa
     unsigned actbits = 0u;  // bit c: constraint lane + 32 c is active
     int q = 0, a_i = -1;    // active set size; this lane's active constraint (lane < q)
     double u_i = 0.0;       // its multiplier
+    double rd = 1.0, rdi = 1.0;  // its diagonal entry of R and the reciprocal
+    double gs = 0.0, gx = 0.0;   // its coefficient not yet in s; in s, not yet in x
     int iters = 0;
     bool converged = false, overflow = false;
     while (true) {
@@ -640,13 +707,12 @@ __global__ void __launch_bounds__(32 * kIclsGramWarps, 1) k_icls_gram(IclsGramPa
           bestp = ci;
         }
       }
-      for (int o = 16; o > 0; o >>= 1) {
-        const double ob = __shfl_xor_sync(kFull, best, o);
-        const int op = __shfl_xor_sync(kFull, bestp, o);
-        if (op >= 0 && (bestp < 0 || ob < best || (ob == best && op < bestp))) {
-          best = ob;
-          bestp = op;
-        }
+      const int arg = warp_argmin(best, bestp >= 0);
+      if (arg >= 0) {  // equal values: the first constraint
+        const double low = __shfl_sync(kFull, best, arg);
+        bestp = static_cast<int>(
+            __reduce_min_sync(kFull, bestp >= 0 && best == low ? static_cast<unsigned>(bestp) : 0xffffffffu));
+        best = low;
       }
       if (bestp < 0) {
         converged = true;
@@ -655,13 +721,15 @@ __global__ void __launch_bounds__(32 * kIclsGramWarps, 1) k_icls_gram(IclsGramPa
       double sp = best;
       const double gpp = __ldg(p.Gam + static_cast<size_t>(bestp) * mp + bestp);
       bool stop = false;
+      double tp = 0.0;  // p's own coefficient
       while (true) {  // inner loop: drop blocking constraints until p is added
         // d1 = R^-T Gamma[A, p] (forward substitution by columns of R^T)
         double d1 = (lane < q) ? __ldg(p.Gam + static_cast<size_t>(a_i) * mp + bestp) : 0.0;
         for (int k = 0; k < q; ++k) {
-          const double dk = __shfl_sync(kFull, d1, k) / R[k * kIclsGramRs + k];
+          const double rk = R[k * kIclsGramRs + lane];
+          const double dk = __shfl_sync(kFull, quotient(d1, rd, rdi), k);
           if (lane == k) d1 = dk;
-          else if (lane > k && lane < q) d1 = fma(-R[k * kIclsGramRs + lane], dk, d1);
+          else if (lane > k && lane < q) d1 = fma(-rk, dk, d1);
         }
         double dd = d1 * d1;
         for (int o = 16; o > 0; o >>= 1) dd += __shfl_xor_sync(kFull, dd, o);
@@ -669,57 +737,31 @@ __global__ void __launch_bounds__(32 * kIclsGramWarps, 1) k_icls_gram(IclsGramPa
         // r = R^-1 d1 (back substitution by columns, icls.rs:331-341)
         double rr = d1;
         for (int i = q - 1; i >= 0; --i) {
-          const double ri = __shfl_sync(kFull, rr, i) / R[i * kIclsGramRs + i];
+          const double rk = R[lane * kIclsGramRs + i];
+          const double ri = __shfl_sync(kFull, quotient(rr, rd, rdi), i);
           if (lane == i) rr = ri;
-          else if (lane < i) rr = fma(-R[lane * kIclsGramRs + i], ri, rr);
+          else if (lane < i) rr = fma(-rk, ri, rr);
         }
-        // step lengths (icls.rs:343-368)
+        // step lengths (icls.rs:343-368): t1 from the lanes of the active set,
+        // t2 from lane 31 in the same division
+        const bool cand = lane < q && rr > p.tol;
+        const double num = lane == 31 ? -sp : u_i, den = lane == 31 ? zn : (cand ? rr : 1.0);
+        const double ratio = num / den;
+        const double r2 = __shfl_sync(kFull, ratio, 31);
         double t1 = INFINITY;
         int drop = -1;
-        if (lane < q && rr > p.tol) {
-          t1 = u_i / rr;
-          drop = lane;
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-          const double ot = __shfl_xor_sync(kFull, t1, o);
-          const int od = __shfl_xor_sync(kFull, drop, o);
-          if (od >= 0 && (drop < 0 || ot < t1 || (ot == t1 && od < drop))) {
-            t1 = ot;
-            drop = od;
-          }
-        }
-        const double t2 = (zn > p.tol) ? -sp / zn : INFINITY;
+        drop = warp_argmin(ratio, cand && ratio < INFINITY);
+        if (drop >= 0) t1 = __shfl_sync(kFull, ratio, drop);
+        const double t2 = (zn > p.tol) ? r2 : INFINITY;
         const double t = fmin(t1, t2);
         if (!isfinite(t)) {
           stop = true;  // infeasible
           break;
         }
         if (lane < q) u_i -= t * rr;
-        // s += t (Gamma[:, p] - Gamma[:, A] r), x += t (u_p - U_A r) (= L^-T of x~'s step)
-        {
-          double ds[CPL], dx[RPL];
-          const double* gp = p.Gam + static_cast<size_t>(bestp) * mp + lane;
-          const double* wp = p.UT + static_cast<size_t>(bestp) * Kp + lane;
-#pragma unroll
-          for (int c = 0; c < CPL; ++c) ds[c] = __ldg(gp + 32 * c);
-#pragma unroll
-          for (int c = 0; c < RPL; ++c) dx[c] = (lane + 32 * c < Kp) ? __ldg(wp + 32 * c) : 0.0;
-          for (int i = 0; i < q; ++i) {
-            const double ri = __shfl_sync(kFull, rr, i);
-            const int ai = __shfl_sync(kFull, a_i, i);
-            const double* ga = p.Gam + static_cast<size_t>(ai) * mp + lane;
-            const double* wa = p.UT + static_cast<size_t>(ai) * Kp + lane;
-#pragma unroll
-            for (int c = 0; c < CPL; ++c) ds[c] = fma(-ri, __ldg(ga + 32 * c), ds[c]);
-#pragma unroll
-            for (int c = 0; c < RPL; ++c)
-              if (lane + 32 * c < Kp) dx[c] = fma(-ri, __ldg(wa + 32 * c), dx[c]);
-          }
-#pragma unroll
-          for (int c = 0; c < CPL; ++c) s[c] = fma(t, ds[c], s[c]);
-#pragma unroll
-          for (int c = 0; c < RPL; ++c) xt[c] = fma(t, dx[c], xt[c]);
-        }
+        // s += t (Gamma[:, p] - Gamma[:, A] r), x += t (u_p - U_A r): recorded
+        tp += t;
+        if (lane < q) gs = fma(-t, rr, gs);
         if (isfinite(t2) && t == t2) {
           // full step: constraint p joins the active set
           if (q >= qcap) {
@@ -729,19 +771,34 @@ __global__ void __launch_bounds__(32 * kIclsGramWarps, 1) k_icls_gram(IclsGramPa
           }
           if (lane < q) R[lane * kIclsGramRs + q] = d1;
           if (lane == q) {
-            R[q * kIclsGramRs + q] = sqrt(zn);
+            rd = sqrt(zn);
+            rdi = 1.0 / rd;
+            R[q * kIclsGramRs + q] = rd;
             a_i = bestp;
             u_i = t;
+            gs = tp;
+            gx = 0.0;
           }
           if (lane == (bestp & 31)) actbits |= 1u << (bestp >> 5);
           __syncwarp();
           q += 1;
+          icls_gram_move(s, p.Gam, mp, lane, q, gs, a_i);
+          gx += gs;
+          gs = 0.0;
+          tp = 0.0;
           break;
         }
         // partial step: the blocking constraint leaves (icls.rs:385-398, 465-501)
         sp += t * zn;
         const int kd = drop;
         const int dropped = __shfl_sync(kFull, a_i, kd);
+        {
+          const double gd = __shfl_sync(kFull, gs, kd);
+          const double* gp = p.Gam + static_cast<size_t>(dropped) * mp + lane;
+#pragma unroll
+          for (int c = 0; c < CPL; ++c) s[c] = fma(gd, __ldg(gp + 32 * c), s[c]);
+          icls_gram_x(xt, p.UT, Kp, lane, __shfl_sync(kFull, gx, kd) + gd, dropped);
+        }
         if (lane < q) {  // each lane shifts its own row of R left past column kd
           for (int col = kd; col < q - 1; ++col) R[lane * kIclsGramRs + col] = R[lane * kIclsGramRs + col + 1];
           R[lane * kIclsGramRs + q - 1] = 0.0;
@@ -751,7 +808,7 @@ __global__ void __launch_bounds__(32 * kIclsGramWarps, 1) k_icls_gram(IclsGramPa
           const double aa = R[i * kIclsGramRs + i], bb = R[(i + 1) * kIclsGramRs + i];
           if (bb == 0.0) continue;
           const double rn = sqrt(aa * aa + bb * bb);
-          const double cg = aa / rn, sg = bb / rn;
+          const double rni = 1.0 / rn, cg = quotient(aa, rn, rni), sg = quotient(bb, rn, rni);
           __syncwarp();
           for (int col = i + lane; col < q - 1; col += 32) {
             const double ri = R[i * kIclsGramRs + col], rj = R[(i + 1) * kIclsGramRs + col];
@@ -760,23 +817,37 @@ __global__ void __launch_bounds__(32 * kIclsGramWarps, 1) k_icls_gram(IclsGramPa
           }
           __syncwarp();
         }
-        {  // entry kd leaves the active list and the multipliers
+        {  // entry kd leaves the active list, the multipliers and the coefficients
           const double un = __shfl_down_sync(kFull, u_i, 1);
+          const double sn = __shfl_down_sync(kFull, gs, 1);
+          const double xn = __shfl_down_sync(kFull, gx, 1);
           const int an = __shfl_down_sync(kFull, a_i, 1);
           if (lane >= kd && lane < q - 1) {
             u_i = un;
             a_i = an;
+            gs = sn;
+            gx = xn;
+            rd = R[lane * kIclsGramRs + lane];
+            rdi = 1.0 / rd;
           } else if (lane == q - 1) {
-            u_i = 0.0;
+            u_i = gs = gx = 0.0;
             a_i = -1;
+            rd = rdi = 1.0;
           }
         }
         if (lane == (dropped & 31)) actbits &= ~(1u << (dropped >> 5));
         __syncwarp();
         q -= 1;
       }
-      if (stop) break;
+      if (stop) {  // p did not join
+        if (tp != 0.0) icls_gram_x(xt, p.UT, Kp, lane, tp, bestp);
+        break;
+      }
     }
+    gx += gs;
+#pragma unroll 2
+    for (int i = 0; i < q; ++i)
+      icls_gram_x(xt, p.UT, Kp, lane, __shfl_sync(kFull, gx, i), __shfl_sync(kFull, a_i, i));
     executed += static_cast<unsigned long long>(iters - 1);
 
 #pragma unroll
