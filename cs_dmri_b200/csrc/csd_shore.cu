@@ -3242,7 +3242,7 @@ int csd_shore_microstructure(csd_handle* h, const float* coefficients, int64_t X
       d_dirs = h->pdir.as<float>();
     }
     h->pconst.ensure(sizeof(csd::MicroConsts));
-    csd::k_micro_consts<<<1, 1, 0, st>>>(radial_order, zeta, h->pconst.as<csd::MicroConsts>());
+    csd::k_micro_consts<<<1, csd::kMicroMaxBlocks, 0, st>>>(radial_order, zeta, h->pconst.as<csd::MicroConsts>());
     CSD_LAUNCH();
     // unit scales (io/microstructure.rs:162-173)
     const bool um = units == 0;

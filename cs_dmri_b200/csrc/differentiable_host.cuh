@@ -200,7 +200,7 @@ const csd::MicroConsts* micro_consts(csd_handle* h, int radial_order, double zet
     throw Error{CSD_ERR_INVALID, "radial order must be even and at most 14 for the RTOP constants"};
   if (!(h->adjconst.p && h->adjconst_order == radial_order && h->adjconst_zeta == zeta)) {
     h->adjconst.ensure(sizeof(csd::MicroConsts));
-    csd::k_micro_consts<<<1, 1, 0, h->stream>>>(radial_order, zeta, h->adjconst.as<csd::MicroConsts>());
+    csd::k_micro_consts<<<1, csd::kMicroMaxBlocks, 0, h->stream>>>(radial_order, zeta, h->adjconst.as<csd::MicroConsts>());
     CSD_LAUNCH();
     h->adjconst_order = radial_order;
     h->adjconst_zeta = zeta;

@@ -12,13 +12,17 @@
 
 namespace csd {
 
-constexpr int kApplyTile = 16;  // voxels per tile of k_apply_rows
+constexpr int kApplyTile = 16;   // voxels per tile of k_apply_rows
+constexpr int kApplyVoxels = 8;  // voxels per thread: one read of AT each k for all of them
 
 // out[v, i] = f32( sum_k AT[k, i] * c[v, k] ) for every voxel v of the
 // volume, the products summed in k order in FP64 (the reference's gemv
 // column order, synth.rs:60 / models.rs:238-243).  A voxel outside `mask`
 // (if given), or with every coefficient exactly zero when `skip_zero` is set
-// (synth.rs:55-58), is written as zeros.  AT is K x R, R contiguous.
+// (synth.rs:55-58), is written as zeros.  AT is K x R, R contiguous.  Bound by
+// the load pipe: with one voxel a thread two loads for every product (32,768
+// voxels, K = 72, R = 259 and 28: 405 us), with eight a load of AT serves eight
+// (220 us).
 __global__ void __launch_bounds__(256) k_apply_rows(const float* __restrict__ coeffs, int64_t nvox, int K,
                                                     const double* __restrict__ AT, int R,
                                                     const uint8_t* __restrict__ mask, int skip_zero,
@@ -43,16 +47,24 @@ __global__ void __launch_bounds__(256) k_apply_rows(const float* __restrict__ co
       act[v] = a;
     }
     __syncthreads();
-    for (int idx = threadIdx.x; idx < nv * R; idx += blockDim.x) {
-      const int v = idx / R, i = idx - v * R;
-      float o = 0.0f;
-      if (act[v]) {
-        double acc = 0.0;
-        const double* cv = sc + v * K;
-        for (int k = 0; k < K; ++k) acc = __dadd_rn(acc, __dmul_rn(__ldg(AT + static_cast<size_t>(k) * R + i), cv[k]));
-        o = static_cast<float>(acc);
+    constexpr int VB = kApplyVoxels;
+    for (int idx = threadIdx.x; idx < (nv + VB - 1) / VB * R; idx += blockDim.x) {
+      const int w = idx / R, i = idx - w * R;
+      double acc[VB];
+#pragma unroll
+      for (int j = 0; j < VB; ++j) acc[j] = 0.0;
+      const double* cv = sc + w * VB * K;  // rows past nv hold an earlier tile's values, not stored
+#pragma unroll 4
+      for (int k = 0; k < K; ++k) {
+        const double a = __ldg(AT + static_cast<size_t>(k) * R + i);
+#pragma unroll
+        for (int j = 0; j < VB; ++j) acc[j] = __dadd_rn(acc[j], __dmul_rn(a, cv[j * K + k]));
       }
-      out[v0 * R + idx] = o;
+#pragma unroll
+      for (int j = 0; j < VB; ++j) {
+        const int v = w * VB + j;
+        if (v < nv) out[(v0 + v) * R + i] = act[v] ? static_cast<float>(acc[j]) : 0.0f;
+      }
     }
     __syncthreads();
   }
@@ -159,32 +171,39 @@ __device__ double dev_rtpp_kappa(unsigned j, unsigned l) {
   return pre * sum;
 }
 
-// One thread fills the constants (a few hundred scalars, once per call).
-__global__ void k_micro_consts(int radial_order, double zeta, MicroConsts* __restrict__ mc) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
-  mc->radial_order = radial_order;
-  mc->zeta = zeta;
-  int start = 0, nb = 0;
+// The constants (a few hundred scalars, once per call), one thread per (n, l)
+// block (at most kMicroMaxBlocks): a chain of math calls each, 56 us together
+// at order 6 against 361 in one thread.
+__global__ void __launch_bounds__(kMicroMaxBlocks) k_micro_consts(int radial_order, double zeta,
+                                                                MicroConsts* __restrict__ mc) {
+  // this thread's block (n, l) is found first, so that the lanes evaluate theirs together
+  int start = 0, nb = 0, bn = -1, bl = 0, bstart = 0;
   for (int n = 0; n <= radial_order; ++n)
     for (int l = 0; l <= n; l += 2) {
-      if (l == 0) mc->n00[n] = start;
-      mc->blk_start[nb] = start;
-      mc->blk_len[nb] = 2 * l + 1;
-      mc->blk_l[nb] = l;
-      const unsigned j = static_cast<unsigned>(n - l + 1);
-      mc->rtap_k[nb] = dev_rtap_kappa(j, l);
-      mc->rtpp_k[nb] = dev_rtpp_kappa(j, l);
-      // alpha(n, l) (microstructure.rs:272-278)
-      const double sign = ((l / 2) % 2 == 0) ? 1.0 : -1.0;
-      const double num = 2.0 * CUDART_PI * pow(zeta, 1.5) * lanczos_gamma(static_cast<double>(n) + 1.5);
-      const double den = pow(2.0, static_cast<double>(l)) * dev_factorial(n - l);
-      mc->alpha[nb] = sign * sqrt(num / den);
+      if (nb == static_cast<int>(threadIdx.x)) {
+        bn = n;
+        bl = l;
+        bstart = start;
+      }
       start += 2 * l + 1;
       ++nb;
     }
-  mc->K = start;
-  mc->n_blocks = nb;
-  for (int n = 0; n <= radial_order; ++n) {
+  if (bn >= 0) {
+    const int b = threadIdx.x;
+    if (bl == 0) mc->n00[bn] = bstart;
+    mc->blk_start[b] = bstart;
+    mc->blk_len[b] = 2 * bl + 1;
+    mc->blk_l[b] = bl;
+    const unsigned j = static_cast<unsigned>(bn - bl + 1);
+    mc->rtap_k[b] = dev_rtap_kappa(j, bl);
+    mc->rtpp_k[b] = dev_rtpp_kappa(j, bl);
+    // alpha(n, l) (microstructure.rs:272-278)
+    const double sign = ((bl / 2) % 2 == 0) ? 1.0 : -1.0;
+    const double num = 2.0 * CUDART_PI * pow(zeta, 1.5) * lanczos_gamma(static_cast<double>(bn) + 1.5);
+    const double den = pow(2.0, static_cast<double>(bl)) * dev_factorial(bn - bl);
+    mc->alpha[b] = sign * sqrt(num / den);
+  }
+  for (int n = threadIdx.x; n <= radial_order; n += blockDim.x) {
     const double g = lanczos_gamma(n + 1.5), f = dev_factorial(n);
     mc->r0[n] = dev_kappa(zeta, n, 0) * dev_gen_laguerre(n, 0.5, 0.0);
     mc->rtop_w[n] = sqrt(16.0 * CUDART_PI * pow(zeta, 1.5) * g / f);
@@ -194,6 +213,11 @@ __global__ void k_micro_consts(int radial_order, double zeta, MicroConsts* __res
     mc->gam[n] = g;
     mc->fact[n] = f;
   }
+  if (threadIdx.x != 0) return;
+  mc->radial_order = radial_order;
+  mc->zeta = zeta;
+  mc->K = start;
+  mc->n_blocks = nb;
   mc->qiv_pre = 6.0 * sqrt(2.0 * CUDART_PI) * pow(zeta, 2.5);
   const double mu = 1.0 / (2.0 * CUDART_PI * sqrt(zeta));
   mc->rtap_pre = 1.0 / (mu * mu);

@@ -50,3 +50,24 @@ def test_tikhonov_by_the_refined_inverse(order, n_dirs, lam):
     b = s.cpu().numpy().astype(np.float64) @ M
     bound = np.abs(c) @ np.abs(H) + np.abs(b) + np.abs(s.cpu().numpy()) @ np.abs(M)
     assert (np.abs(c @ H - b) <= len(nl) * 2.0 ** -53 * bound).all()
+
+
+@pytest.mark.parametrize("order", [2, 6, 8])
+@pytest.mark.parametrize("v", [1, 7, 8, 9, 16, 17, 2385])
+def test_predicted_signal_at_ragged_volumes(order, v, oracle):
+    """Eight voxels a thread, sixteen a tile: every sum is in coefficient
+    order without fused operations, so the signals equal the oracle's to one
+    rounding of a design entry per term; zero voxels stay zero."""
+    from cs_dmri_b200 import shore_predict
+    from cs_dmri_b200.phantom import make_phantom
+    ph = make_phantom((2, 2, 2), seed=5)
+    K = sum(2 * l + 1 for n in range(order + 1) for l in range(0, n + 1, 2))
+    rng = np.random.default_rng(v)
+    c = rng.normal(size=(v, 1, 1, K)).astype(np.float32)
+    c[v // 2] = 0.0
+    kw = dict(big_delta=ph.big_delta, small_delta=ph.small_delta)
+    got = shore_predict(c, order, 700.0, ph.bvals, ph.bvecs, **kw)
+    want = oracle.shore_predict(c, order, 700.0, ph.bvals, ph.bvecs, **kw)
+    assert not got[v // 2].any()
+    scale = np.abs(want).max()
+    np.testing.assert_allclose(got, want, rtol=2.4e-7, atol=1e-9 * max(scale, 1e-30))
