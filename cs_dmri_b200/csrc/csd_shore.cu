@@ -344,7 +344,7 @@ struct csd_handle {
   // converged-optimum modes: the TF32 B operand (per table), the iterate,
   // per-voxel KKT residuals, overflow / failure lists, counters
   // [batches, error, n_overflow, n_failed, rounds, kkt max bits, n_failed2]
-  DevBuf gtf32, x32, kktv, kktovf, kktfail, kktstat;
+  DevBuf gtf32, x32, kktv, kktovf, kktwide, kktfail, kktstat;
   uint64_t gtf32_key = 0;
   bool gtf32_valid = false;
   cudaEvent_t kev[5] = {};
@@ -1195,6 +1195,21 @@ void launch_polish_t(csd_handle* h, const csd::PolishParams& q, int warps, int64
   CSD_LAUNCH();
 }
 
+template <int RPH>
+void launch_polish_half_t(csd_handle* h, const csd::PolishParams& q) {
+  constexpr int THREADS = 256;
+  const size_t smem = sizeof(double) * (THREADS / 16) * static_cast<size_t>(csd::polish_half_doubles(q.Kp));
+  auto* kern = csd::k_l1_polish_half<RPH>;
+  CSD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  int per_sm = 0;
+  CSD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, THREADS, smem));
+  const int64_t need = (q.n_work + THREADS / 16 - 1) / (THREADS / 16);
+  const int blocks = static_cast<int>(
+      std::max<int64_t>(1, std::min<int64_t>(static_cast<int64_t>(h->num_sms) * std::max(per_sm, 1), need)));
+  kern<<<blocks, THREADS, smem, h->stream>>>(q);
+  CSD_LAUNCH();
+}
+
 // Supports of up to 32 coefficients keep their vectors in one register per
 // lane; the passes with room for all K coefficients take ceil(K / 32).
 void launch_polish(csd_handle* h, const csd::PolishParams& q, int warps, int64_t items) {
@@ -1211,6 +1226,15 @@ void launch_polish(csd_handle* h, const csd::PolishParams& q, int warps, int64_t
     throw Error{CSD_ERR_INVALID, "the converged-optimum polish is built for radial orders <= 6"};
   }
 }
+
+// Whether the first polish takes two voxels per warp (k_l1_polish_half: fewer
+// instructions a voxel, a longer round, and a second launch for supports above
+// sixteen).  Whole fits with 32 iterations, one / two voxels per warp, N = 259:
+//   order 6: 32,000 voxels 536 / 551 us, 64,000 voxels 802 / 784 us, 128,000
+//            voxels 1,303 / 1,211 us, 299,200 voxels 2,662 / 2,382 us
+//   order 4: 32,000 voxels 409 / 424 us, 64,000 voxels 594 / 580 us, 299,200
+//            voxels 1,840 / 1,546 us
+bool polish_half(const csd_handle* h, int64_t n_work) { return h->Kp <= 80 && n_work > 384 * h->num_sms; }
 
 void launch_fista_kkt(csd_handle* h, int MT, const csd::FistaParams& p);
 
@@ -1305,9 +1329,9 @@ void launch_fista_kkt(csd_handle* h, int MT, const csd::FistaParams& p) {
   // stat: [0] tensor batches, [1] tensor error, [2] first-pass overflows,
   // [3] failures (the fallback's list), [4] rounds, [5] largest KKT residual
   // (bits), [6] uncertified, [7] unused overflow count
-  h->kktstat.ensure(8 * sizeof(unsigned long long));
+  h->kktstat.ensure(10 * sizeof(unsigned long long));
   auto* stat = h->kktstat.as<unsigned long long>();
-  CSD_CUDA(cudaMemsetAsync(stat, 0, 8 * sizeof(unsigned long long), st));
+  CSD_CUDA(cudaMemsetAsync(stat, 0, 10 * sizeof(unsigned long long), st));
   h->kktv.ensure(sizeof(double) * std::max<int64_t>(V, 1));
   h->kktovf.ensure(sizeof(int64_t) * std::max<int64_t>(p.n_work, 1));
   h->kktfail.ensure(sizeof(int64_t) * std::max<int64_t>(p.n_work, 1));
@@ -1397,6 +1421,19 @@ void launch_fista_kkt(csd_handle* h, int MT, const csd::FistaParams& p) {
   pp.round_total = stat + 4;
   pp.kkt_max_bits = stat + 5;
   pp.n_uncertified = stat + 6;  // non-finite inputs (failures go to the fallback list)
+  if (polish_half(h, p.n_work)) {
+    h->kktwide.ensure(sizeof(int64_t) * static_cast<size_t>(p.n_work));
+    csd::PolishParams ph = pp;
+    ph.overflow = h->kktwide.as<int64_t>();
+    ph.n_overflow = stat + 8;
+    ph.queue = stat + 9;
+    if (Kp <= 32)
+      launch_polish_half_t<2>(h, ph);
+    else
+      launch_polish_half_t<5>(h, ph);
+    pp.list = h->kktwide.as<int64_t>();
+    pp.list_len = stat + 8;
+  }
   launch_polish(h, pp, 8, p.n_work);
   csd::PolishParams po = pp;
   po.list = h->kktovf.as<int64_t>();
@@ -2829,7 +2866,7 @@ void csd_destroy(csd_handle* h) {
                     &h->iota, &h->adjW, &h->adjovf, &h->adjstat, &h->adjconst, &h->hinv, &h->hmat,
                     &h->gdtab, &h->gdq, &h->tuneB, &h->tuneX, &h->tuneIt, &h->tuneConv, &h->tuneQ,
                     &h->schedY, &h->schedPend, &h->schedKey, &h->schedOrder, &h->schedCnt,
-                    &h->schedD, &h->schedU, &h->schedN, &h->ppark, &h->gtf32, &h->x32, &h->kktv, &h->kktovf,
+                    &h->schedD, &h->schedU, &h->schedN, &h->ppark, &h->gtf32, &h->x32, &h->kktv, &h->kktovf, &h->kktwide,
                     &h->kktfail, &h->kktstat};
   for (auto s : h->pipe)
     if (s) cudaStreamSynchronize(s);
