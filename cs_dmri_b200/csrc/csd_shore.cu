@@ -695,7 +695,7 @@ void launch_fista_t(csd_handle* h, const csd::FistaParams& p) {
 
 // Two-pass schedule: a fit is split at iteration sched_cap() when it has at
 // least kSchedMinWaves voxels per FISTA slot (fewer: the slowest voxels start
-// in the first wave anyway) and max_iter is above twice the cap.  The slot
+// in the first wave anyway, and hybrid_fista splits it) and max_iter is above twice the cap.  The slot
 // count of the call's grid sets the scale.  The handle option
 // CSD_OPT_FISTA_SCHEDULE turns it off (0) or sets the cap (>= 2).
 constexpr int kSchedCap = 80;

@@ -235,7 +235,7 @@ typedef struct csd_fit_timing {
   float ms_total;       /* device time from first to last kernel */
   int32_t launches;     /* kernels launched by the fit */
   float ms_solve_kernel;/* duration of the dominant solve kernel alone */
-  double tensor_flops;  /* FP64 tensor-core FLOPs the FISTA launches executed */
+  double tensor_flops;  /* FP64 tensor-core FLOPs the FISTA launches executed (0 where sparse warps serve) */
   float ms_mixed_kernel;/* the mixed-precision FISTA kernel alone (0 in FP64) */
   double int8_tensor_ops;      /* int8 tensor-core ops it issued (2 per MAC) */
   uint64_t fp64_rerun_voxels;  /* voxels the stop-decision guard re-ran in FP64 */
@@ -265,10 +265,13 @@ typedef struct csd_fit_timing {
 int csd_last_timing(const csd_handle* h, csd_fit_timing* out);
 
 /* Tuning options of a handle (they never change a result's meaning):
- *   CSD_OPT_FISTA_SHAPE     FP64 FISTA kernel: 0 = the per-table autotuned
- *                           choice (default), 12 or 16 warps per CTA of the
- *                           DMMA kernel, 1 = the register kernel; every
- *                           shape computes the same iterates
+ *   CSD_OPT_FISTA_SHAPE     FP64 FISTA kernel: 0 = the library's choice by
+ *                           size and radial order (default: sparse warps,
+ *                           the DMMA kernel with the per-table autotuned
+ *                           shape, or both in turn; alpha paths fused), 12
+ *                           or 16 warps per CTA of the DMMA kernel, 1 = the
+ *                           register kernel; every shape computes the same
+ *                           iterates
  *   CSD_OPT_FISTA_SCHEDULE  0 = single-pass FISTA; 1 = the two-pass
  *                           schedule where it applies (default); a value
  *                           >= 2 also sets its cap (iteration of the first
