@@ -694,9 +694,8 @@ void launch_fista_t(csd_handle* h, const csd::FistaParams& p) {
 }
 
 // Two-pass schedule: a fit is split at iteration sched_cap() when it has at
-// least kSchedMinWaves voxels per FISTA slot (fewer: the slowest voxels start
-// in the first wave anyway, and hybrid_fista splits it) and max_iter is above twice the cap.  The slot
-// count of the call's grid sets the scale.  The handle option
+// least kSchedMinWaves voxels per FISTA slot of a full grid (fewer: hybrid_fista
+// splits it) and max_iter is above twice the cap.  The handle option
 // CSD_OPT_FISTA_SCHEDULE turns it off (0) or sets the cap (>= 2).
 constexpr int kSchedCap = 80;
 
@@ -707,6 +706,7 @@ int sched_cap(const csd_handle* h) {
 }
 constexpr int64_t kSchedMinWaves = 4;
 constexpr size_t kSchedSlotBytes = 4096;  // count (8 B), bucket counts, bucket cursors
+constexpr size_t kSchedNnzAt = 3072;       // of a slot: non-zero count of the parked y, then the lengths of the second pass
 constexpr int kSchedSlots = 16;
 
 // Single-pass FISTA for the lifetime of the guard.
@@ -738,24 +738,35 @@ void ensure_sched(csd_handle* h, int64_t V) {
 // grid holds `slots` voxels at a time.
 void launch_fista_sparse(csd_handle* h, const csd::FistaParams& p);
 
-// From one to kHybridWaves waves of DMMA slots the second pass runs on the
-// sparse kernel: 80 iterations at the DMMA warps' throughput (most voxels of a
-// large alpha end there), then the slowest voxels first on warps that take a
-// sixth of the time an iteration.  Per volume fit, N = 259, against a single
-// DMMA pass and the two passes both on DMMA slots:
-//   order 6, alpha 0.01:  38,760 voxels 2.42 ms (single 3.22), 77,520 voxels
-//     4.35 (two DMMA passes 5.27), 124,032 voxels 5.81 (6.34), 193,800 voxels
-//     8.77 (8.64), 299,432 voxels 13.4 (12.6)
-//   order 6, alpha 0.05:  38,760 voxels 0.44 ms (sparse alone 0.47), 65,892
-//     voxels 0.57 (0.63)
-//   order 4, alpha 0.01:  38,760 voxels 1.09 ms (1.33), 124,032 voxels 2.15
-//     (2.42), 310,080 voxels 4.86 (4.65)
+// From dmma_voxels() (at order 6 kChooseVoxels per SM) to kHybridWaves waves of
+// DMMA slots the two passes go to two kernels: the first 80 iterations to the DMMA slots, at their
+// throughput (most voxels of a large alpha end there), then the slowest voxels
+// first to sparse warps, which take a sixth of the time an iteration, or to
+// DMMA slots again where the parked y are dense (PassChoice): a sparse warp pays
+// for every non-zero entry, a DMMA slot takes 118 SM cycles a voxel-iteration at
+// the most.  Volume fits, N = 259, second pass on sparse warps / on DMMA slots,
+// with the parked voxels' mean number of non-zero entries (alpha 0.01, 0.005,
+// 0.002, 0.001, alpha-ratio 1e-3):
+//   order 6              12 of 72     18          29          38          49
+//      9,500 voxels ms  1.06/2.26  2.22/4.11   4.56/6.05   6.63/6.18   9.88/6.68
+//     18,900            1.45/2.86  3.15/5.09   7.15/7.65   10.5/7.85   15.1/8.89
+//     40,000            2.84/4.08  6.29/6.78   14.5/12.5   21.3/15.0   30.7/18.3
+//    150,000            6.81/6.93  19.2/16.3   48.4/33.8   73.1/41.0    109/57.0
+//   order 4              11 of 29     16          21          23          25
+//     15,000 voxels ms  0.67/1.04  1.20/1.72   2.43/2.27   2.86/2.36   3.93/3.09
+//     40,000            1.07/1.57  2.12/2.40   5.43/3.48   6.51/3.71   9.54/6.14
+//    150,000            2.57/2.77  6.63/4.77   18.8/8.96   22.8/10.0   35.0/19.6
+// The lines cross at kDenseBase + scale / (voxels per SM + kDenseLead) entries
+// (48 / 38 / 29 / 21 / 14 of 72 at 30 / 64 / 128 / 270 / 1,000 per SM).
+// Above kHybridWaves waves sparse warps no longer gain where they are ahead
+// (order 6, alpha 0.01, 299,432 voxels 13.4 / 12.6 ms).
 constexpr int64_t kHybridWaves = 8;
+constexpr int kDenseBase = 10, kDenseLead = 72;
 
 bool hybrid_fista(const csd_handle* h, const csd::FistaParams& p, int64_t slots) {
   const int cap = sched_cap(h);
   return (h->K == 29 || h->K == 72) && h->opt_shape == 0 && cap > 0 && h->sched_off == 0 && p.cap == 0 &&
-         !p.n_work_dev && p.max_iter > 2 * cap && p.n_work >= slots && p.n_work < kHybridWaves * slots;
+         !p.n_work_dev && p.max_iter > 2 * cap && p.n_work < kHybridWaves * slots;
 }
 
 template <class Go>
@@ -776,6 +787,7 @@ void launch_fista_sched(csd_handle* h, const csd::FistaParams& p, int64_t slots,
   auto* n_pend = reinterpret_cast<unsigned long long*>(cnt);
   auto* hist = reinterpret_cast<unsigned*>(cnt + 8);
   unsigned* cursor = hist + csd::kSchedBins;
+  auto* nnz = reinterpret_cast<unsigned long long*>(cnt + kSchedNnzAt);
   int64_t* pend = h->schedPend.as<int64_t>() + h->sched_base;
   float* key = h->schedKey.as<float>() + h->sched_base;
   int64_t* order = h->schedOrder.as<int64_t>() + h->sched_base;
@@ -787,10 +799,23 @@ void launch_fista_sched(csd_handle* h, const csd::FistaParams& p, int64_t slots,
   q1.pend = pend;
   q1.pend_key = key;
   q1.n_pend = n_pend;
+  csd::PassChoice choice{};
+  if (hybrid) {
+    choice.Y = q1.Y;
+    choice.Kp = h->Kp;
+    choice.nnz = nnz;
+    choice.n_dmma = nnz + 1;
+    choice.n_sparse = nnz + 2;
+    choice.base = kDenseBase;
+    choice.lead = kDenseLead;
+    choice.scale = h->K == 29 ? 1900 : 3800;
+    choice.sms = h->num_sms;
+  }
   go(q1);
-  csd::k_sched_hist<<<h->num_sms, 256, 0, st>>>(key, n_pend, hist, p.iter_total ? p.iter_total + 2 : nullptr);
+  csd::k_sched_hist<<<h->num_sms, 256, 0, st>>>(pend, key, n_pend, hist, p.iter_total ? p.iter_total + 2 : nullptr,
+                                                choice);
   CSD_LAUNCH();
-  csd::k_sched_order<<<h->num_sms, csd::kSchedBins, 0, st>>>(pend, key, n_pend, hist, cursor, order, p.queue);
+  csd::k_sched_order<<<h->num_sms, csd::kSchedBins, 0, st>>>(pend, key, n_pend, hist, cursor, order, p.queue, choice);
   CSD_LAUNCH();
   csd::FistaParams q2 = q1;
   q2.resume = 1;
@@ -799,10 +824,12 @@ void launch_fista_sched(csd_handle* h, const csd::FistaParams& p, int64_t slots,
   q2.n_work_dev = n_pend;
   q2.pend = nullptr;
   q2.pend_key = nullptr;
-  if (hybrid)
+  if (hybrid) {  // one of the two has the whole list, the other returns at once
+    q2.n_work_dev = choice.n_sparse;
     launch_fista_sparse(h, q2);
-  else
-    go(q2);
+    q2.n_work_dev = choice.n_dmma;
+  }
+  go(q2);
 }
 
 template <int MT, int WARPS, bool NONNEG>
@@ -815,12 +842,16 @@ void launch_fista_v3_n(csd_handle* h, const csd::FistaParams& p) {
   int per_sm = 0;
   CSD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * WARPS, smem));
   per_sm = std::max(per_sm, 1);
-  const int64_t warps_needed = (p.n_work + 7) / 8;
+  // a short list spreads over the SMs, on at least four warps (which stage G)
+  // to a CTA
+  const int64_t need = (p.n_work + 7) / 8;
   const int sms = h->sm_cap > 0 ? std::min(h->sm_cap, h->num_sms) : h->num_sms;
-  const int64_t blocks = std::max<int64_t>(
-      1, std::min<int64_t>(static_cast<int64_t>(sms) * per_sm, (warps_needed + WARPS - 1) / WARPS));
-  launch_fista_sched(h, p, blocks * WARPS * 8, [&](const csd::FistaParams& q) {
-    kern<<<static_cast<unsigned>(blocks), 32 * WARPS, smem, h->stream>>>(q);
+  const int64_t need_sm = (need + sms - 1) / sms;
+  const int64_t ctas = std::min<int64_t>(per_sm, std::max<int64_t>(1, (need_sm + WARPS - 1) / WARPS));
+  const int warps = static_cast<int>(std::min<int64_t>(WARPS, std::max<int64_t>(4, (need_sm + ctas - 1) / ctas)));
+  const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>(sms * ctas, (need + warps - 1) / warps));
+  launch_fista_sched(h, p, static_cast<int64_t>(sms) * per_sm * WARPS * 8, [&](const csd::FistaParams& q) {
+    kern<<<static_cast<unsigned>(blocks), 32 * warps, smem, h->stream>>>(q);
     CSD_LAUNCH();
   });
 }
@@ -862,27 +893,64 @@ void launch_fista_sparse_p(csd_handle* h, const csd::FistaParams& p) {
 }
 
 // Whether a fit of n_work voxels takes the sparse kernel alone (handle option
-// CSD_OPT_FISTA_SHAPE left at 0; every kernel computes the same iterates).
-// Measured per volume fit on B200, sparse against k_fista_v3, N = 259, alpha
-// 0.01:
-//   order 4:  15,504 voxels 0.68 / 1.33 ms, 300,763 voxels 6.41 / 5.25 ms
-//   order 6:   4,000 voxels 0.84 / 2.80 ms, 15,504 voxels 1.26 / 2.38 ms,
-//            125,000 voxels 6.97 / 6.25 ms
-//   order 8:  32,000 voxels 4.56 / 6.87 ms, 300,763 voxels 33.2 / 47.5 ms
-// A warp of k_fista_v3 takes 2 us an iteration for its eight voxels and the
-// slowest voxel's up to 1,000 iterations set a small fit's time; a sparse warp
-// takes 0.3 us.  From one wave of DMMA slots the first iterations of a fit are
-// bound by throughput, where the DMMA slots are ahead (alpha 0.05, 19
-// iterations, 65,892 voxels: 0.63 / 0.57 ms at order 6, 0.41 / 0.38 at order
-// 4), and hybrid_fista takes over; with the schedule off (a walk that launches
-// point by point) sparse warps up to four waves.  At order 8 G's tiles do not
-// fit in shared memory beside the slots' vectors and 9 % of y's entries are
-// non-zero: always sparse.
+// CSD_OPT_FISTA_SHAPE left at 0; every kernel computes the same iterates):
+// fewer than dmma_voxels(), where the slowest voxel's up to 1,000
+// iterations set the time and one takes 0.3 us on a sparse warp, 1.2-4 us on a
+// DMMA one.  Volume fits, N = 259, sparse warps alone / first pass on DMMA slots
+// (the second as hybrid_fista chooses):
+//   order 6:  4,736 voxels alpha 0.05 0.25 / 0.28 ms, 0.01 0.84 / 0.91,
+//     alpha-ratio 1e-3 5.7 / 4.3; 9,500 voxels 0.29 / 0.31, 1.06 / 1.06, 10.6 /
+//     6.7; 15,000 voxels 0.33 / 0.33, 1.27 / 1.16, 16.0 / 8.6
+//   order 4:  9,500 voxels 0.22 / 0.24, 0.55 / 0.64, 2.9 / 2.5; 15,000 voxels
+//     0.25 / 0.26, 0.70 / 0.67, 4.2 / 3.1
+// The lines lie where a sparse alpha loses 5 % at most, and a dense one is not
+// yet behind k_fista_v3 in 16-warp CTAs (order 6 8.2 ms, order 4 3.3 ms).
+// At order 8 G's tiles do not fit in shared memory beside the slots' vectors:
+// always sparse (32,000 voxels, alpha 0.01 3.4 ms against 11.9 with G read
+// through the caches, alpha-ratio 1e-3 72 / 101 ms).
+int64_t dmma_voxels(const csd_handle* h) { return static_cast<int64_t>(h->K == 29 ? 80 : 56) * h->num_sms; }
+
 bool sparse_fista(const csd_handle* h, int64_t n_work) {
   if (h->K == 145) return true;
-  if (h->opt_shape != 0 || (h->K != 29 && h->K != 72)) return false;
-  const int64_t slots = static_cast<int64_t>(h->num_sms) * 16 * 8;
-  return n_work < (h->sched_off > 0 ? kSchedMinWaves : 1) * slots;
+  return h->opt_shape == 0 && (h->K == 29 || h->K == 72) && n_work < dmma_voxels(h);
+}
+
+// A single pass on sparse warps or on DMMA slots, chosen by the alphas
+// (k_choose_by_alpha): DMMA where the iterates are dense, and where there are
+// many voxels of few iterations.  For dmma_voxels() to four waves of voxels in
+// the caller's order (slowest first by its own account, which the two passes
+// would not keep), and at order 6 for up to kChooseVoxels per SM in any order:
+// two passes cost a sparse alpha 0.14 ms there (8,300 voxels, alpha 0.01: 1.06
+// ms against 0.93 on sparse warps), the choice 0.01 ms.
+// Fits of DifferentiableShore, N = 259, alpha_max about 0.33, sparse warps / DMMA
+// slots in ms by alpha:
+//   order 6             0.05       0.02       0.01       0.005      0.002      0.001
+//     9,500 voxels   0.26/0.28  0.43/0.63  0.88/2.45  1.87/4.01  4.34/5.32  6.50/5.92
+//    25,000          0.38/0.35  0.75/0.79  1.60/3.03  3.66/5.09  9.07/7.42  13.8/7.95
+//    75,000          0.72/0.56  1.74/1.34  3.95/3.80  10.3/7.55  25.9/15.9  39.2/19.4
+//   order 4
+//    19,000          0.25/0.22  0.37/0.37  0.76/1.36  1.25/1.84  2.82/2.18  3.41/2.35
+//    75,000          0.43/0.35  0.95/0.68  1.73/1.65  4.07/2.49  10.5/4.23  12.6/4.71
+// The dense line lies at alpha / alpha_max of 0.0025 / 0.0055 / 0.018 / 0.032 and
+// the other at 0.27 / 0.13 / 0.05 / 0.045 at 64 / 128 / 338 / 507 voxels per SM.
+constexpr int64_t kChooseVoxels = 72;
+
+bool chosen_fista(const csd_handle* h, const csd::FistaParams& p) {
+  if (h->opt_shape != 0 || (h->K != 29 && h->K != 72) || p.n_work_dev) return false;
+  if (h->sched_off > 0 && p.list) return p.n_work < kSchedMinWaves * h->num_sms * 16 * 8;
+  return h->K == 72 && p.n_work < kChooseVoxels * h->num_sms;
+}
+
+// The lengths of the two kernels' lists, sparse then DMMA.
+void choose_by_alpha(csd_handle* h, const csd::FistaParams& p, const unsigned long long*& n) {
+  h->schedCnt.ensure(kSchedSlotBytes * kSchedSlots);
+  auto* len = reinterpret_cast<unsigned long long*>(static_cast<char*>(h->schedCnt.p) +
+                                                    kSchedSlotBytes * h->sched_slot + kSchedNnzAt) + 1;
+  const double per_sm = static_cast<double>(p.n_work) / h->num_sms;
+  const double low = 3.6e-5 * per_sm * (1.0 + per_sm / 700.0), high = std::max(0.045, 17.0 / per_sm);
+  csd::k_choose_by_alpha<<<1, 1024, 0, h->stream>>>(p, h->K, h->Kp, low, high, len + 1, len);
+  CSD_LAUNCH();
+  n = len;
 }
 
 // One voxel per warp has the shorter iteration, two share the reads of G's
@@ -1105,9 +1173,11 @@ void launch_fista_mixed(csd_handle* h, const csd::FistaParams& p) {
     q1.n_pend = n_pend;
     csd::k_fista_i8<<<grid, THREADS, smem, st>>>(q1);
     CSD_LAUNCH();
-    csd::k_sched_hist<<<h->num_sms, 256, 0, st>>>(key, n_pend, hist, p.iter_total ? p.iter_total + 2 : nullptr);
+    csd::k_sched_hist<<<h->num_sms, 256, 0, st>>>(pend, key, n_pend, hist, p.iter_total ? p.iter_total + 2 : nullptr,
+                                                  csd::PassChoice{});
     CSD_LAUNCH();
-    csd::k_sched_order<<<h->num_sms, csd::kSchedBins, 0, st>>>(pend, key, n_pend, hist, cursor, order, p.queue);
+    csd::k_sched_order<<<h->num_sms, csd::kSchedBins, 0, st>>>(pend, key, n_pend, hist, cursor, order, p.queue,
+                                                               csd::PassChoice{});
     CSD_LAUNCH();
     csd::MixedParams q2 = q1;
     q2.resume = 1;
@@ -1500,26 +1570,8 @@ void launch_fista_kkt(csd_handle* h, int MT, const csd::FistaParams& p) {
   h->kkt_iter_add += static_cast<unsigned long long>(p.n_work) * static_cast<unsigned long long>(k1);
 }
 
-void launch_fista(csd_handle* h, int MT, const csd::FistaParams& p) {
-  if ((h->precision == CSD_PRECISION_MIXED_KKT || h->precision == CSD_PRECISION_FP64_KKT) && p.max_iter > 0) {
-    launch_fista_kkt(h, MT, p);
-    return;
-  }
-  if (h->precision == CSD_PRECISION_MIXED && MT * 8 == csd::i8::KC && p.max_iter > 0) {
-    launch_fista_mixed(h, p);
-    return;
-  }
-  if (p.max_iter <= 0) {
-    // An empty iteration loop: the warm start (or zero) is the result, with
-    // 0 iterations and not converged (fista.rs:89-143 with max_iter = 0).
-    csd::k_fista_noop<<<grid1(p.n_work * (h->Kp + 1)), 256, 0, h->stream>>>(p, h->Kp);
-    CSD_LAUNCH();
-    return;
-  }
-  if (sparse_fista(h, p.n_work)) {
-    launch_fista_sparse(h, p);
-    return;
-  }
+// The DMMA kernel's shape for the table, or the register kernel.
+void launch_fista_dmma(csd_handle* h, int MT, const csd::FistaParams& p) {
   const int variant = fista_variant(h);
   if (variant == 3 || variant == 4) {
     switch (MT * 8 + variant) {
@@ -1540,6 +1592,37 @@ void launch_fista(csd_handle* h, int MT, const csd::FistaParams& p) {
       throw Error{CSD_ERR_INVALID, "FISTA kernels are built for radial orders 2, 4, 6 and 8 (K <= 145); got K = " +
                                        std::to_string(h->K)};
   }
+}
+
+void launch_fista(csd_handle* h, int MT, const csd::FistaParams& p) {
+  if ((h->precision == CSD_PRECISION_MIXED_KKT || h->precision == CSD_PRECISION_FP64_KKT) && p.max_iter > 0) {
+    launch_fista_kkt(h, MT, p);
+    return;
+  }
+  if (h->precision == CSD_PRECISION_MIXED && MT * 8 == csd::i8::KC && p.max_iter > 0) {
+    launch_fista_mixed(h, p);
+    return;
+  }
+  if (p.max_iter <= 0) {
+    // An empty iteration loop: the warm start (or zero) is the result, with
+    // 0 iterations and not converged (fista.rs:89-143 with max_iter = 0).
+    csd::k_fista_noop<<<grid1(p.n_work * (h->Kp + 1)), 256, 0, h->stream>>>(p, h->Kp);
+    CSD_LAUNCH();
+    return;
+  }
+  if (sparse_fista(h, p.n_work)) {
+    launch_fista_sparse(h, p);
+    return;
+  }
+  if (chosen_fista(h, p)) {  // one of the two kernels has the whole list, the other returns at once
+    csd::FistaParams q = p;
+    choose_by_alpha(h, p, q.n_work_dev);
+    launch_fista_sparse(h, q);
+    ++q.n_work_dev;
+    launch_fista_dmma(h, MT, q);
+    return;
+  }
+  launch_fista_dmma(h, MT, p);
 }
 
 // Whether one row tile of a matrix of `cols` columns fits in shared memory.

@@ -37,6 +37,7 @@ void run_fit_batch(csd_handle* h, const float* d_sig, int64_t V, const HostGtab&
   h->iters.ensure(sizeof(uint32_t) * V);
   h->conv.ensure(V);
   h->queue.ensure(sizeof(unsigned long long));
+  h->schedCnt.ensure(kSchedSlotBytes * kSchedSlots);  // before a capture that gives an order for the first time
   csd::k_iota<<<grid1(V), 256, 0, st>>>(h->vox.as<int64_t>(), V);
   CSD_LAUNCH();
   // Tikhonov with the DMMA product c = P s, as the volume fit does

@@ -524,6 +524,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_fista_v3(FistaParams p) {
   constexpr int KP = 8 * MT, KT = 2 * MT;
   constexpr int G_WORDS = MT * KT * 32;
   extern __shared__ __align__(16) double smem3[];
+  if (p.n_work_dev && *p.n_work_dev == 0) return;
   const double* sG = smem3;                                        // MT * KT * 32 (k_pack_gfrag)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double* ybuf = smem3 + G_WORDS + warp * (2 * KP * 8);           // KP x 8 [k][voxel]
@@ -666,6 +667,59 @@ __global__ void __launch_bounds__(32 * WARPS) k_fista_v3(FistaParams p) {
   if (p.kstep_total && lane == 0) atomicAdd(p.kstep_total, static_cast<unsigned long long>(ksteps));
 }
 
+// The kernel of the second pass, chosen on the device by what pass 1 parked:
+// the DMMA slots take the list (*n_dmma = its length, *n_sparse = 0) when the
+// parked voxels' y (rows of Y) have at least base + scale / (voxels per SM +
+// lead) non-zero entries on average, else the sparse warps do.  The average is
+// over kChoiceSample voxels spread over the list, counted into *nnz.
+struct PassChoice {
+  const double* Y;  // V x Kp; nullptr: no choice
+  int Kp, base, lead, scale, sms;
+  unsigned long long *nnz, *n_dmma, *n_sparse;
+};
+constexpr int kChoiceSample = 4096;
+
+__device__ __forceinline__ long long choice_sample(long long n) { return n < kChoiceSample ? n : kChoiceSample; }
+
+__device__ __forceinline__ bool dense_pass(const PassChoice& c, long long n) {
+  const long long m = choice_sample(n);
+  return (static_cast<long long>(*c.nnz) - c.base * m) * (n + static_cast<long long>(c.lead) * c.sms) >=
+         static_cast<long long>(c.scale) * c.sms * m;
+}
+
+// The kernel of a single pass, chosen by its voxels' alphas relative to
+// alpha_max (||b||_inf / n): sparse warps when that of at least half of a
+// sample of the voxels lies in [low, high], else the DMMA slots.
+constexpr int kAlphaSample = 128;
+
+__global__ void __launch_bounds__(1024) k_choose_by_alpha(FistaParams p, int K, int Kp, double low, double high,
+                                                          unsigned long long* __restrict__ n_dmma,
+                                                          unsigned long long* __restrict__ n_sparse) {
+  __shared__ int within, counted;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) within = counted = 0;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kAlphaSample / 32; ++i) {
+    const int64_t w = (32 * i + warp) * p.n_work / kAlphaSample;
+    const int64_t v = p.list ? p.list[w] : w;
+    double bm = 0.0;
+    for (int k = lane; k < K; k += 32) bm = fmax(bm, fabs(p.B[v * Kp + k]));
+    const double thr = p.alpha_v ? __dmul_rn(p.step, p.alpha_v[v]) : p.thr;
+    for (int o = 16; o > 0; o >>= 1) bm = fmax(bm, __shfl_xor_sync(kFull, bm, o));
+    const double thr_max = bm * p.n_inv * p.step;
+    if (lane == 0 && thr_max > 0.0) {
+      atomicAdd(&counted, 1);
+      if (thr >= low * thr_max && thr <= high * thr_max) atomicAdd(&within, 1);
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  const bool dmma = 2 * within < counted;
+  *n_dmma = dmma ? p.n_work : 0;
+  *n_sparse = dmma ? 0 : p.n_work;
+}
+
 // Order of the second pass of the two-pass FISTA schedule: the voxels that
 // pass 1 parked, largest predicted remaining iteration count first (the ones
 // likely to need the most iterations start first instead of finishing
@@ -682,11 +736,12 @@ __device__ __forceinline__ int sched_bin(float key) {
 }
 
 // hist[b] += keys in bucket b (hist zeroed by the caller); the key count is
-// added to *parked_total (nullable).
-__global__ void __launch_bounds__(256) k_sched_hist(const float* __restrict__ key,
+// added to *parked_total (nullable); the non-zero entries of the choice's
+// sample are counted.
+__global__ void __launch_bounds__(256) k_sched_hist(const int64_t* __restrict__ pend, const float* __restrict__ key,
                                                     const unsigned long long* __restrict__ n_key,
                                                     unsigned* __restrict__ hist,
-                                                    unsigned long long* __restrict__ parked_total) {
+                                                    unsigned long long* __restrict__ parked_total, PassChoice choice) {
   __shared__ unsigned sh[kSchedBins];
   if (*n_key == 0) return;
   if (parked_total && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(parked_total, *n_key);
@@ -696,6 +751,18 @@ __global__ void __launch_bounds__(256) k_sched_hist(const float* __restrict__ ke
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x)
     atomicAdd(&sh[sched_bin(key[i])], 1u);
+  if (choice.Y) {
+    const int lane = threadIdx.x & 31;
+    const int64_t m = choice_sample(n);
+    int nnz = 0;
+    for (int64_t i = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / 32; i < m;
+         i += static_cast<int64_t>(gridDim.x) * blockDim.x / 32) {
+      const double* y = choice.Y + pend[i * n / m] * choice.Kp;
+      for (int k = lane; k < choice.Kp; k += 32) nnz += y[k] != 0.0;
+    }
+    nnz = __reduce_add_sync(kFull, nnz);
+    if (lane == 0 && nnz) atomicAdd(choice.nnz, static_cast<unsigned long long>(nnz));
+  }
   __syncthreads();
   for (int b = threadIdx.x; b < kSchedBins; b += blockDim.x)
     if (sh[b]) atomicAdd(&hist[b], sh[b]);
@@ -704,15 +771,22 @@ __global__ void __launch_bounds__(256) k_sched_hist(const float* __restrict__ ke
 // order[] = pend[] by bucket, highest bucket first.  Block `blk` handles one
 // contiguous segment: it reserves a run in each bucket with one atomic per
 // bucket (cursor zeroed by the caller), then places its entries.  256 threads.
-// The work queue is reset for the pass that follows.
+// The work queue is reset for the pass that follows, and its kernel chosen.
 __global__ void __launch_bounds__(256) k_sched_order(const int64_t* __restrict__ pend, const float* __restrict__ key,
                                                      const unsigned long long* __restrict__ n_key,
                                                      const unsigned* __restrict__ hist, unsigned* __restrict__ cursor,
                                                      int64_t* __restrict__ order,
-                                                     unsigned long long* __restrict__ queue) {
+                                                     unsigned long long* __restrict__ queue, PassChoice choice) {
   __shared__ unsigned scan[kSchedBins], base[kSchedBins], cnt[kSchedBins];
   const int t = threadIdx.x;
-  if (blockIdx.x == 0 && t == 0) *queue = 0;
+  if (blockIdx.x == 0 && t == 0) {
+    *queue = 0;
+    if (choice.Y) {
+      const bool dense = dense_pass(choice, static_cast<long long>(*n_key));
+      *choice.n_dmma = dense ? *n_key : 0;
+      *choice.n_sparse = dense ? 0 : *n_key;
+    }
+  }
   if (*n_key == 0) return;
   // base[b] = entries in buckets above b (inclusive scan over reversed buckets)
   scan[t] = hist[kSchedBins - 1 - t];
