@@ -272,7 +272,11 @@ struct csd_handle {
   // mtfrag), so an L2 fit is the single product c = P s; built with the factor
   DevBuf pfrag, ptmp;
   bool pfrag_valid = false;
-  DevBuf hmat;                // H itself (refinement of the solves)
+  // the same operator transposed (N x Kp) for the apply kernel, where the
+  // right-hand-side kernel does not serve the table
+  DevBuf l2mat;
+  bool l2mat_valid = false;
+  double chol_growth = 0.0;   // max_j H_jj / l_jj^2 of the current factor
   DevBuf hinv;                // H^{-1} of the current factor (L2 adjoint)
   bool hinv_valid = false;
   uint64_t hinv_key = 0;
@@ -428,6 +432,38 @@ void set_err(char* err, size_t len, const std::string& msg) {
 
 void autotune_fista(csd_handle* h);
 void launch_tikhonov(csd_handle* h, const double* B, double* X, int64_t V);
+bool apply_dmma_fits(const csd_handle* h, int cols);
+
+// Whether the explicit operator P = H^-1 M^T of the current factor gives a
+// Tikhonov fit as exact as the factor's two substitutions on b = M^T s.  P does
+// not round b, the larger part of the substitutions' error, but its
+// normal-equation residual grows with the condition of H (scaled by its
+// diagonal), of which H_jj / l_jj^2 is a sign.  Product / substitutions against
+// extended precision (root mean square and largest relative error of 301 voxels,
+// 2,001 at order 4), the residuals in units of 2^-53 (|H||c| + |M|^T|s|) from a
+// float64 model:
+//                          H_jj / l_jj^2   rms              largest          residual
+//   order 8, 259 samples
+//     lambda 0.05               1.0     5.5 / 9.0 e-16   1.6 / 3.3 e-15   5.3 / 6.1
+//     1e-8                       13     3.4 / 4.2 e-14   0.6 / 1.5 e-13   5.0 / 5.2
+//     1e-9                       64                                       8.4 / 5.9
+//     1e-12                   3,400                                        89 / 3.3
+//     0                         6e8                                       967 / 14
+//   order 6, 401, 0.05          1.0     5.1 / 7.1 e-16   1.9 / 2.2 e-15   4.2 / 3.7
+//                 1e-8           15     2.5 / 4.4 e-14   0.6 / 1.3 e-13   4.5 / 4.1
+//   order 4, 515, 0.05          1.0     7.7 / 8.0 e-16   2.5 / 2.8 e-15
+constexpr double kProductGrowth = 32.0;
+bool l2_product_exact(const csd_handle* h) { return h->chol_growth <= kProductGrowth; }
+
+// H^-1 of the current factor from its solves' rows (K rows, stride Kp).
+void keep_hinv(csd_handle* h, const double* rows) {
+  const size_t K = static_cast<size_t>(h->K);
+  h->hinv.ensure(sizeof(double) * K * K);
+  CSD_CUDA(cudaMemcpy2DAsync(h->hinv.p, sizeof(double) * K, rows, sizeof(double) * h->Kp, sizeof(double) * K, K,
+                             cudaMemcpyDeviceToDevice, h->stream));
+  h->hinv_key = h->chol_key;
+  h->hinv_valid = true;
+}
 
 // Build (or reuse) the per-gradient-table device setup.
 void ensure_setup(csd_handle* h, const HostGtab& g, int radial_order, double zeta, bool need_chol,
@@ -445,6 +481,7 @@ void ensure_setup(csd_handle* h, const HostGtab& g, int radial_order, double zet
     h->setup_valid = false;
     h->chol_valid = false;
     h->pfrag_valid = false;
+    h->l2mat_valid = false;
     h->icls_valid = false;
     h->N = N;
     h->K = K;
@@ -530,31 +567,43 @@ void ensure_setup(csd_handle* h, const HostGtab& g, int radial_order, double zet
       const size_t csm = sizeof(double) * static_cast<size_t>(K) * K;
       CSD_CUDA(cudaFuncSetAttribute(csd::k_cholesky, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     static_cast<int>(csm)));
-      h->hmat.ensure(sizeof(double) * Kp * Kp);
-      CSD_CUDA(cudaMemcpyAsync(h->hmat.p, h->A.p, sizeof(double) * Kp * Kp, cudaMemcpyDeviceToDevice, st));
-      csd::k_cholesky<<<1, 256, csm, st>>>(h->A.as<double>(), K, Kp, h->ok.as<int>());
+      csd::k_cholesky<<<1, 256, csm, st>>>(h->A.as<double>(), K, Kp, h->ok.as<int>(), h->scal.as<double>() + 2);
       CSD_LAUNCH();
       int okv = 0;
       CSD_CUDA(cudaMemcpyAsync(&okv, h->ok.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+      CSD_CUDA(cudaMemcpyAsync(&h->chol_growth, h->scal.as<double>() + 2, sizeof(double), cudaMemcpyDeviceToHost, st));
       CSD_CUDA(cudaStreamSynchronize(st));
       if (!okv) throw Error{CSD_ERR_NUMERICAL, "normal-equations matrix should be PD"};
       h->chol_key = ck;
       h->chol_valid = true;
-      // P^T = rows H^-1 m_n of the design rows m_n, by the factor's solves,
-      // then packed like M^T for the right-hand-side kernel
-      h->pfrag_valid = false;
-      if (h->dmma_rhs) {
-        h->ptmp.ensure(2 * sizeof(double) * static_cast<size_t>(N) * Kp);
+      // P^T = rows H^-1 m_n of the design rows m_n, by the factor's solves:
+      // packed like M^T for the right-hand-side kernel, or as it stands, with
+      // the rows of H^-1 from the same launch, for the apply kernel
+      h->pfrag_valid = h->l2mat_valid = false;
+      const bool apply = !h->dmma_rhs && l2_product_exact(h) && apply_dmma_fits(h, N);
+      if (h->dmma_rhs || apply) {
+        const size_t rows = static_cast<size_t>(N) + (apply ? K : 0);
+        h->ptmp.ensure(sizeof(double) * (apply ? 1 : 2) * rows * Kp);
+        if (apply) h->l2mat.ensure(sizeof(double) * rows * Kp);
         double* mpad = h->ptmp.as<double>();
-        double* pt = mpad + static_cast<size_t>(N) * Kp;
+        double* pt = apply ? h->l2mat.as<double>() : mpad + rows * Kp;
         csd::k_pad_rows<<<(N * Kp + 255) / 256, 256, 0, st>>>(h->M.as<double>(), N, K, Kp, mpad);
         CSD_LAUNCH();
-        launch_tikhonov(h, mpad, pt, N);
-        h->pfrag.ensure(sizeof(double) * static_cast<size_t>(h->Np) * Kp);
-        csd::k_pack_afrag<<<(h->Np * Kp + 255) / 256, 256, 0, st>>>(pt, N, K, Kp, 1, Kp, h->Np,
-                                                                    h->pfrag.as<double>());
-        CSD_LAUNCH();
-        h->pfrag_valid = true;
+        if (apply) {
+          csd::k_identity_rows<<<(K * Kp + 255) / 256, 256, 0, st>>>(mpad + static_cast<size_t>(N) * Kp, K, Kp);
+          CSD_LAUNCH();
+        }
+        launch_tikhonov(h, mpad, pt, static_cast<int64_t>(rows));
+        if (apply) {
+          keep_hinv(h, pt + static_cast<size_t>(N) * Kp);
+          h->l2mat_valid = true;
+        } else {
+          h->pfrag.ensure(sizeof(double) * static_cast<size_t>(h->Np) * Kp);
+          csd::k_pack_afrag<<<(h->Np * Kp + 255) / 256, 256, 0, st>>>(pt, N, K, Kp, 1, Kp, h->Np,
+                                                                      h->pfrag.as<double>());
+          CSD_LAUNCH();
+          h->pfrag_valid = true;
+        }
       }
     }
   }
@@ -591,7 +640,7 @@ void ensure_icls_setup(csd_handle* h, int radial_order, double zeta, double eps)
   const size_t csm = sizeof(double) * static_cast<size_t>(K) * K;
   CSD_CUDA(cudaFuncSetAttribute(csd::k_cholesky, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(csm)));
-  csd::k_cholesky<<<1, 256, csm, st>>>(h->Le.as<double>(), K, Kp, h->ok.as<int>());
+  csd::k_cholesky<<<1, 256, csm, st>>>(h->Le.as<double>(), K, Kp, h->ok.as<int>(), nullptr);
   CSD_LAUNCH();
   int okv = 0;
   CSD_CUDA(cudaMemcpyAsync(&okv, h->ok.p, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -1668,41 +1717,47 @@ void launch_rhs_t(csd_handle* h, const float* d_data, int64_t V) {
 }
 
 template <int KP>
-void launch_rhs_dmma_t(csd_handle* h, const float* d_data, int64_t V, float* sig_out, const double* frag,
-                       double* out) {
+void launch_rhs_dmma_t(csd_handle* h, const float* d_data, const int64_t* rows, int64_t V, float* sig_out,
+                       const double* frag, double* out) {
   const size_t smem = sizeof(double) * static_cast<size_t>(h->Np) * KP + sizeof(float) * 8 * 8 * (h->Np + 4);
   CSD_CUDA(cudaFuncSetAttribute(csd::k_rhs_dmma<KP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(smem)));
   const int64_t groups = (V + 7) / 8;
   const int blocks = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(h->num_sms, (groups + 7) / 8)));
-  csd::k_rhs_dmma<KP><<<blocks, 256, smem, h->stream>>>(d_data, h->vox.as<int64_t>(), V, h->N, h->Np, frag, out,
-                                                        sig_out);
+  csd::k_rhs_dmma<KP><<<blocks, 256, smem, h->stream>>>(d_data, rows, V, h->N, h->Np, frag, out, sig_out);
   CSD_LAUNCH();
 }
 
-// Whether c = P s with the Tikhonov operator serves an L2 fit of the table.
-bool l2_operator_ready(const csd_handle* h) { return h->dmma_rhs && h->pfrag_valid; }
+// Whether c = P s with the Tikhonov operator serves an L2 fit of the table; the
+// others solve by the factor from b (k_tikhonov).
+bool l2_operator_ready(const csd_handle* h) { return (h->dmma_rhs && h->pfrag_valid) || h->l2mat_valid; }
 
-// b = M^T s for every masked voxel into h->B; or, with `l2_out` set, c = P s
-// (l2_operator_ready) into it.  A design that does not fit one CTA's shared
-// memory (radial order 8, or more than 288 samples) goes through the apply
-// kernel's chunks of row tiles, with the same sums: 32,000 voxels at order 8,
-// N = 259, 277 us on k_rhs's FMAs.
-void launch_rhs(csd_handle* h, const float* d_data, int64_t V, float* sig_out = nullptr, double* l2_out = nullptr) {
+// b = M^T s for every masked voxel (row rows[v] of d_data) into h->B; or, with
+// `l2_out` set, c = P s (l2_operator_ready) into it.  A design that does not fit
+// one CTA's shared memory (radial order 8, or more than 288 samples) goes
+// through the apply kernel's chunks of row tiles, with the same sums: 32,000
+// voxels at order 8, N = 259, 277 us on k_rhs's FMAs.  c = P s there: 3,001
+// voxels at order 8 355 us by the substitutions, 31 us by the product.
+void launch_rhs(csd_handle* h, const float* d_data, const int64_t* rows, int64_t V, float* sig_out = nullptr,
+                double* l2_out = nullptr) {
   if (h->dmma_rhs) {
     const double* f = l2_out ? h->pfrag.as<double>() : h->mtfrag.as<double>();
     double* o = l2_out ? l2_out : h->B.as<double>();
     switch (h->Kp) {
-      case 8: launch_rhs_dmma_t<8>(h, d_data, V, sig_out, f, o); return;
-      case 32: launch_rhs_dmma_t<32>(h, d_data, V, sig_out, f, o); return;
-      case 72: launch_rhs_dmma_t<72>(h, d_data, V, sig_out, f, o); return;
+      case 8: launch_rhs_dmma_t<8>(h, d_data, rows, V, sig_out, f, o); return;
+      case 32: launch_rhs_dmma_t<32>(h, d_data, rows, V, sig_out, f, o); return;
+      case 72: launch_rhs_dmma_t<72>(h, d_data, rows, V, sig_out, f, o); return;
       default: break;
     }
   }
-  if (l2_out) throw Error{CSD_ERR_INVALID, "the Tikhonov operator product needs the DMMA right-hand-side kernel"};
+  if (l2_out) {
+    launch_apply_dmma<float>(h, h->l2mat.as<double>(), h->Kp, h->K, h->N, d_data, h->N, rows, V, l2_out, nullptr, h->Kp,
+                             h->Kp);
+    return;
+  }
   if (apply_dmma_fits(h, h->N)) {
-    launch_apply_dmma<float>(h, h->M.as<double>(), h->K, h->K, h->N, d_data, h->N, h->vox.as<int64_t>(), V,
-                             h->B.as<double>(), nullptr, h->Kp, h->Kp);
+    launch_apply_dmma<float>(h, h->M.as<double>(), h->K, h->K, h->N, d_data, h->N, rows, V, h->B.as<double>(), nullptr,
+                             h->Kp, h->Kp);
     return;
   }
   switch (h->Kp) {
@@ -1732,27 +1787,6 @@ void launch_tikhonov(csd_handle* h, const double* B, double* X, int64_t V) {
     case 5: go(csd::k_tikhonov<5>); break;
     default: throw Error{CSD_ERR_INVALID, "Tikhonov kernel supports K <= 160"};
   }
-}
-
-void ensure_hinv(csd_handle* h);
-
-// H c = b for every voxel where the operator product does not apply (order 8,
-// long tables): the inverse's product with one step of refinement, c = H^-1 b,
-// c += H^-1 (b - H c), whose normal-equation residual is that of the
-// substitution (k_tikhonov: 2 K serial steps a voxel, each a division and a
-// shuffle).  Measured at 3,001 voxels, order 8: 355 -> 65 us; relative error
-// against a 64-bit solve over orders 6 and 8, 150-515 samples, lambda 1e-8 to
-// 0.05: see the bounds in the differentiable fit's tests.
-void solve_l2(csd_handle* h, const double* B, double* X, int64_t V) {
-  if (V <= 0) return;
-  ensure_hinv(h);
-  const int K = h->K, Kp = h->Kp;
-  h->adjW.ensure(sizeof(double) * static_cast<size_t>(V) * Kp);
-  double* R = h->adjW.as<double>();
-  const double *Hi = h->hinv.as<double>(), *H = h->hmat.as<double>();
-  launch_apply_dmma<double>(h, Hi, K, K, K, B, Kp, nullptr, V, X, nullptr, Kp, Kp);
-  launch_apply_dmma<double>(h, H, Kp, K, K, X, Kp, nullptr, V, R, nullptr, Kp, Kp, B, -1.0);
-  launch_apply_dmma<double>(h, Hi, K, K, K, R, Kp, nullptr, V, X, nullptr, Kp, Kp, X, 1.0);
 }
 
 void launch_epilogue_ffma(csd_handle* h, const csd::EpilogueParams& p) {
@@ -2151,10 +2185,10 @@ FitInfo run_fit(csd_handle* h, const float* d_data, const uint8_t* d_mask, int64
     // `d_data` aliases pinned host memory: read each masked row once over the
     // bus and keep a compact device copy for every later pass.
     h->sig.ensure(sizeof(float) * static_cast<size_t>(V) * N);
-    launch_rhs(h, d_data, V, h->sig.as<float>(), rhs_out);
+    launch_rhs(h, d_data, h->vox.as<int64_t>(), V, h->sig.as<float>(), rhs_out);
     h->sig_compact = h->sig.as<float>();
   } else {
-    launch_rhs(h, d_data, V, nullptr, rhs_out);
+    launch_rhs(h, d_data, h->vox.as<int64_t>(), V, nullptr, rhs_out);
   }
   record(h, 2);
 
@@ -2235,7 +2269,7 @@ FitInfo run_fit(csd_handle* h, const float* d_data, const uint8_t* d_mask, int64
   } else if (spec->regularization == CSD_REG_L2) {
     kind = 2;
     record(h, 6);
-    if (!l2_operator) solve_l2(h, h->B.as<double>(), h->X.as<double>(), V);
+    if (!l2_operator) launch_tikhonov(h, h->B.as<double>(), h->X.as<double>(), V);
     record(h, 7);
     it_final = nullptr;
     CSD_CUDA(cudaMemsetAsync(h->conv.p, 1, V, st));
@@ -2285,10 +2319,19 @@ FitInfo run_fit(csd_handle* h, const float* d_data, const uint8_t* d_mask, int64
           // Tikhonov reference RSS per voxel (src/fit.rs:436-438).
           h->Xl2.ensure(sizeof(double) * V * Kp);
           h->rss_l2.ensure(sizeof(double) * V);
-          if (l2_operator_ready(h) && !data_on_host)  // one product, as the L2 fit
-            launch_rhs(h, d_data, V, nullptr, h->Xl2.as<double>());
-          else
-            solve_l2(h, h->B.as<double>(), h->Xl2.as<double>(), V);
+          // the same product, or the same solve, for host and device volumes
+          if (l2_operator_ready(h) && l2_product_exact(h)) {
+            const int64_t* rows = h->vox.as<int64_t>();
+            if (h->sig_compact) {
+              h->iota.ensure(sizeof(int64_t) * V);
+              csd::k_iota<<<grid1(V), 256, 0, st>>>(h->iota.as<int64_t>(), V);
+              CSD_LAUNCH();
+              rows = h->iota.as<int64_t>();
+            }
+            launch_rhs(h, h->sig_compact ? h->sig_compact : d_data, rows, V, nullptr, h->Xl2.as<double>());
+          } else {
+            launch_tikhonov(h, h->B.as<double>(), h->Xl2.as<double>(), V);
+          }
           csd::EpilogueParams rp = ep;
           rp.X = h->Xl2.as<double>();
           rp.scatter = false;
@@ -2946,7 +2989,7 @@ void csd_destroy(csd_handle* h) {
                     &h->pbest, &h->psel, &h->pact, &h->palpha_sel, &h->pit_sel, &h->pconv_sel,
                     &h->palpha_fb, &h->pit_fb, &h->pconv_fb, &h->pcode, &h->gdig, &h->gfexp, &h->flagged,
                     &h->mixstat, &h->pcoef, &h->pmat, &h->pout, &h->pgt, &h->pgv, &h->pdir, &h->pconst,
-                    &h->iota, &h->adjW, &h->adjovf, &h->adjstat, &h->adjconst, &h->hinv, &h->hmat,
+                    &h->iota, &h->adjW, &h->adjovf, &h->adjstat, &h->adjconst, &h->hinv, &h->l2mat,
                     &h->gdtab, &h->gdq, &h->tuneB, &h->tuneX, &h->tuneIt, &h->tuneConv, &h->tuneQ,
                     &h->schedY, &h->schedPend, &h->schedKey, &h->schedOrder, &h->schedCnt,
                     &h->schedD, &h->schedU, &h->schedN, &h->ppark, &h->gtf32, &h->x32, &h->kktv, &h->kktovf, &h->kktwide,

@@ -42,7 +42,7 @@ void run_fit_batch(csd_handle* h, const float* d_sig, int64_t V, const HostGtab&
   CSD_LAUNCH();
   // Tikhonov with the DMMA product c = P s, as the volume fit does
   const bool l2_operator = !is_l1 && l2_operator_ready(h);
-  launch_rhs(h, d_sig, V, nullptr, l2_operator ? h->X.as<double>() : nullptr);
+  launch_rhs(h, d_sig, h->vox.as<int64_t>(), V, nullptr, l2_operator ? h->X.as<double>() : nullptr);
   if (is_l1) {
     ensure_mom(h, spec->max_iter);
     if (d_warm) {
@@ -78,7 +78,7 @@ void run_fit_batch(csd_handle* h, const float* d_sig, int64_t V, const HostGtab&
     if (d_iters)
       CSD_CUDA(cudaMemcpyAsync(d_iters, h->iters.p, sizeof(uint32_t) * V, cudaMemcpyDeviceToDevice, st));
   } else {
-    if (!l2_operator) solve_l2(h, h->B.as<double>(), h->X.as<double>(), V);
+    if (!l2_operator) launch_tikhonov(h, h->B.as<double>(), h->X.as<double>(), V);
     if (d_iters) {
       csd::k_fill_u32<<<grid1(V), 256, 0, st>>>(d_iters, V, 1u);
       CSD_LAUNCH();
@@ -145,11 +145,7 @@ void ensure_hinv(csd_handle* h) {
   csd::k_identity_rows<<<(K * Kp + 255) / 256, 256, 0, st>>>(id, K, Kp);
   CSD_LAUNCH();
   launch_tikhonov(h, id, rows, K);
-  h->hinv.ensure(sizeof(double) * static_cast<size_t>(K) * K);
-  CSD_CUDA(cudaMemcpy2DAsync(h->hinv.p, sizeof(double) * K, rows, sizeof(double) * Kp, sizeof(double) * K, K,
-                             cudaMemcpyDeviceToDevice, st));
-  h->hinv_key = h->chol_key;
-  h->hinv_valid = true;
+  keep_hinv(h, rows);
 }
 
 // L2 adjoint: w = H^{-1} gc (the rows of H^{-1} are its columns, so they are

@@ -166,13 +166,19 @@ __global__ void k_lipschitz(const double* __restrict__ G, int Kp, int N, int max
 // Kp x Kp matrix, one CTA.  Writes 0 to *ok_out if A is not positive definite
 // (the reference panics there, src/solver/tikhonov.rs:44).  The accumulation
 // order of every entry is the left-looking order k = 0, 1, ..., so results
-// match a sequential LL^T factorisation.
-__global__ void k_cholesky(double* __restrict__ A, int K, int Kp, int* __restrict__ ok_out) {
+// match a sequential LL^T factorisation.  max_j A_jj / l_jj^2 goes to *growth_out
+// (nullable).
+__global__ void k_cholesky(double* __restrict__ A, int K, int Kp, int* __restrict__ ok_out,
+                           double* __restrict__ growth_out) {
   extern __shared__ double sA[];
   __shared__ int s_ok;
+  __shared__ unsigned long long s_growth;
   const int tid = threadIdx.x, nt = blockDim.x;
   for (int i = tid; i < K * K; i += nt) sA[i] = A[(i / K) * Kp + (i % K)];
-  if (tid == 0) s_ok = 1;
+  if (tid == 0) {
+    s_ok = 1;
+    s_growth = 0;
+  }
   __syncthreads();
   for (int j = 0; j < K; ++j) {
     if (tid == 0) {
@@ -191,6 +197,14 @@ __global__ void k_cholesky(double* __restrict__ A, int K, int Kp, int* __restric
       if (k <= i) sA[i * K + k] = __dsub_rn(sA[i * K + k], __dmul_rn(sA[i * K + j], sA[k * K + j]));
     }
     __syncthreads();
+  }
+  if (growth_out) {
+    for (int j = tid; j < K; j += nt) {
+      const double l = sA[j * K + j], g = A[j * Kp + j] / (l * l);
+      atomicMax(&s_growth, static_cast<unsigned long long>(__double_as_longlong(g > 0.0 ? g : 0.0)));  // orders as its bits
+    }
+    __syncthreads();
+    if (tid == 0) *growth_out = __longlong_as_double(static_cast<long long>(s_growth));
   }
   for (int i = tid; i < Kp * Kp; i += nt) {
     const int r = i / Kp, c = i % Kp;
