@@ -276,7 +276,8 @@ def shore_fit_device(data, mask, bvals, bvecs, *, coefficients=None, stream=None
     res = _abi.FitResult()
     res.coefficients = coefficients.data_ptr()
     err = C.create_string_buffer(4096)
-    s = stream.cuda_stream if stream is not None else torch.cuda.current_stream(data.device).cuda_stream
+    # torch's default stream has the handle 0, which the library takes as its own, unordered stream: 1 is cudaStreamLegacy
+    s = (stream if stream is not None else torch.cuda.current_stream(data.device)).cuda_stream or 1
     code = lib.csd_shore_fit_volume_device(_abi.handle(device), data.data_ptr(), m8.data_ptr(), X, Y, Z,
                                            C.byref(g), C.byref(spec), C.byref(res), C.c_void_p(s), err, len(err))
     del keep
