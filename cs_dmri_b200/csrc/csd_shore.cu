@@ -1346,14 +1346,26 @@ void launch_polish(csd_handle* h, const csd::PolishParams& q, int warps, int64_t
   }
 }
 
-// Whether the first polish takes two voxels per warp (k_l1_polish_half: fewer
+// Whether the first polish may take two voxels per warp (k_l1_polish_half: fewer
 // instructions a voxel, a longer round, and a second launch for supports above
-// sixteen).  Whole fits with 32 iterations, one / two voxels per warp, N = 259:
+// sixteen; k_choose_polish then looks at the starting supports).  Whole fits with
+// 32 iterations, alpha 0.01, N = 259, one / two voxels per warp:
 //   order 6: 32,000 voxels 536 / 551 us, 64,000 voxels 802 / 784 us, 128,000
 //            voxels 1,303 / 1,211 us, 299,200 voxels 2,662 / 2,382 us
 //   order 4: 32,000 voxels 409 / 424 us, 64,000 voxels 594 / 580 us, 299,200
 //            voxels 1,840 / 1,546 us
-bool polish_half(const csd_handle* h, int64_t n_work) { return h->Kp <= 80 && n_work > 384 * h->num_sms; }
+// Non-negative fits at order 6 gain nothing (32 iterations, alpha 0.01: 60,000
+// voxels 729 / 768 us, 300,000 2,274 / 2,250; FP64 iterations 3,579 / 3,758).
+bool polish_half(const csd_handle* h, const csd::FistaParams& p) {
+  return !h->kkt_tuning && h->Kp <= 80 && !(p.non_negative && h->Kp > 32) && p.n_work > 384 * h->num_sms;
+}
+
+// Of kPolishSample starting supports, those above sixteen up to which two voxels
+// per warp are taken.  300,000 voxels, 32 iterations, two / one per warp, with the
+// share of wide supports:
+//   order 6:  2 % 2.40 / 2.70 ms, 29 % 3.54 / 3.59, 71 % 5.63 / 5.27
+//   order 4: 14 % 2.03 / 2.31 ms, 49 % 2.97 / 2.99, 99 % 5.24 / 5.02
+int half_wide_limit(const csd_handle* h) { return csd::kPolishSample * (h->Kp <= 32 ? 8 : 5) / 16; }
 
 void launch_fista_kkt(csd_handle* h, int MT, const csd::FistaParams& p);
 
@@ -1363,7 +1375,12 @@ void launch_fista_kkt(csd_handle* h, int MT, const csd::FistaParams& p);
 // synthetic batch (73,728 single-tensor voxels on the table's own b-values,
 // alpha 0.01) with 16, 24, 32 and 48 iterations, once untimed and once timed,
 // and the fastest count serves the table's fits.  Every count ends at the
-// certified optimum, so the choice changes the time, not the result.
+// certified optimum, so the choice changes the time, not the result.  The batch is
+// polished one voxel per warp: with two, 24, 32 and 48 TF32 iterations at order 6
+// took 0.584 ms each and noise chose among them, while denser fits need the
+// iterations (300,000 voxels, 24 / 32 / 48 of them: alpha 0.02 1.88 / 1.94 / 2.13
+// ms, alpha 0.01 2.47 / 2.40 / 2.45, alpha 0.005 6.0 / 5.3 / 4.6, alpha 0.002 66 /
+// 40 / 25).
 void autotune_kkt(csd_handle* h, int MT, bool non_negative) {
   static constexpr int kCand[4] = {16, 24, 32, 48};
   const uint64_t key = h->setup_key ^ (0x9E3779B97F4A7C15ull * (1 + h->precision + 4 * (non_negative ? 1 : 0)));
@@ -1447,10 +1464,12 @@ void launch_fista_kkt(csd_handle* h, int MT, const csd::FistaParams& p) {
   const int k1 = h->opt_kkt_iters > 0 ? h->opt_kkt_iters : h->kkt_iters_used;
   // stat: [0] tensor batches, [1] tensor error, [2] first-pass overflows,
   // [3] failures (the fallback's list), [4] rounds, [5] largest KKT residual
-  // (bits), [6] uncertified, [7] unused overflow count
-  h->kktstat.ensure(10 * sizeof(unsigned long long));
+  // (bits), [6] uncertified, [7] unused overflow count, [8] supports above
+  // sixteen, [9] the two-voxel polish's queue, [10] and [11] the voxels of the
+  // two forms of the first polish
+  h->kktstat.ensure(12 * sizeof(unsigned long long));
   auto* stat = h->kktstat.as<unsigned long long>();
-  CSD_CUDA(cudaMemsetAsync(stat, 0, 10 * sizeof(unsigned long long), st));
+  CSD_CUDA(cudaMemsetAsync(stat, 0, 12 * sizeof(unsigned long long), st));
   h->kktv.ensure(sizeof(double) * std::max<int64_t>(V, 1));
   h->kktovf.ensure(sizeof(int64_t) * std::max<int64_t>(p.n_work, 1));
   h->kktfail.ensure(sizeof(int64_t) * std::max<int64_t>(p.n_work, 1));
@@ -1540,9 +1559,12 @@ void launch_fista_kkt(csd_handle* h, int MT, const csd::FistaParams& p) {
   pp.round_total = stat + 4;
   pp.kkt_max_bits = stat + 5;
   pp.n_uncertified = stat + 6;  // non-finite inputs (failures go to the fallback list)
-  if (polish_half(h, p.n_work)) {
+  if (polish_half(h, p)) {  // one of the two kernels has the voxels, the other none
     h->kktwide.ensure(sizeof(int64_t) * static_cast<size_t>(p.n_work));
+    csd::k_choose_polish<<<1, 1024, 0, st>>>(pp, half_wide_limit(h), stat + 10, stat + 11);
+    CSD_LAUNCH();
     csd::PolishParams ph = pp;
+    ph.list_len = stat + 10;
     ph.overflow = h->kktwide.as<int64_t>();
     ph.n_overflow = stat + 8;
     ph.queue = stat + 9;
@@ -1550,6 +1572,9 @@ void launch_fista_kkt(csd_handle* h, int MT, const csd::FistaParams& p) {
       launch_polish_half_t<2>(h, ph);
     else
       launch_polish_half_t<5>(h, ph);
+    csd::PolishParams pw = pp;
+    pw.list_len = stat + 11;
+    launch_polish(h, pw, 8, p.n_work);
     pp.list = h->kktwide.as<int64_t>();
     pp.list_len = stat + 8;
   }

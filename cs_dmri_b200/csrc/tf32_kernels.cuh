@@ -719,6 +719,36 @@ __global__ void __launch_bounds__(256, 4) k_l1_polish(PolishParams p) {
   if (p.round_total && lane == 0) atomicAdd(p.round_total, rounds_sum);  // every lane holds the warp's count
 }
 
+// Whether the first polish takes two voxels per warp (*n_half = n_work, *n_full =
+// 0) or one: two when at most `limit` of kPolishSample sampled starting supports
+// hold more than sixteen coefficients.
+constexpr int kPolishSample = 128;
+
+__global__ void __launch_bounds__(1024) k_choose_polish(PolishParams p, int limit,
+                                                        unsigned long long* __restrict__ n_half,
+                                                        unsigned long long* __restrict__ n_full) {
+  __shared__ int wide;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) wide = 0;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kPolishSample / 32; ++i) {
+    const int64_t w = (32 * i + warp) * p.n_work / kPolishSample;
+    const int64_t v = p.list ? p.list[w] : w;
+    int n = 0;
+    for (int j = lane; j < p.K; j += 32) {
+      const double s0 = p.S32 ? static_cast<double>(p.S32[v * p.Kp + j]) : p.S64[v * p.Kp + j];
+      n += s0 > 0.0 || (s0 < 0.0 && !p.non_negative);
+    }
+    n = __reduce_add_sync(0xffffffffu, n);
+    if (lane == 0 && n > 16) atomicAdd(&wide, 1);
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  *n_half = wide > limit ? 0 : p.n_work;
+  *n_full = wide > limit ? p.n_work : 0;
+}
+
 // The same method with two voxels per warp, sixteen lanes each, for supports
 // of up to sixteen: row i of G_SS and of its factor in lane i's registers (the
 // trailing update reads the column by shuffles), the forward substitution
