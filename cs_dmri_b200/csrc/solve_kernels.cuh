@@ -434,14 +434,16 @@ __device__ __forceinline__ unsigned dmma_fista_step(const double* sG, double* yb
   // A k-step whose four y entries are exactly zero for all eight voxels adds
   // only zeros (soft thresholding keeps most of y at 0): only the live ones run
   // (the few k-steps of small orders unrolled, their fragments loaded ahead).
+  // Order 2's two k-steps always run: their marks cost more than the products.
+  constexpr bool MARKS = MT > 1;
   if constexpr (MT <= 4) {
-    ksteps = __popc(live[0] & ((1u << KT) - 1u));
+    ksteps = MARKS ? __popc(live[0] & ((1u << KT) - 1u)) : KT;
     double bf[KT];
 #pragma unroll
     for (int kt = 0; kt < KT; ++kt) bf[kt] = ybuf[(4 * kt + q) * 8 + g];
 #pragma unroll
     for (int kt = 0; kt < KT; ++kt) {
-      if (!((live[0] >> kt) & 1u)) continue;
+      if (MARKS && !((live[0] >> kt) & 1u)) continue;
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt) dmma_m8n8k4(acc[mt][0], acc[mt][1], sG[(mt * KT + kt) * 32 + lane], bf[kt]);
     }
@@ -480,11 +482,12 @@ __device__ __forceinline__ unsigned dmma_fista_step(const double* sG, double* yb
       x[mt][j] = xn;
     }
     *reinterpret_cast<double2*>(&ybuf[row * 8 + 2 * q]) = make_double2(yo[0], yo[1]);
-    if ((__double_as_longlong(yo[0]) | __double_as_longlong(yo[1])) != 0) live[mt / 16] |= 1u << (2 * (mt % 16));
+    if (MARKS && (__double_as_longlong(yo[0]) | __double_as_longlong(yo[1])) != 0) live[mt / 16] |= 1u << (2 * (mt % 16));
   }
   // rows 8 mt .. 8 mt + 3 (lanes 0-15) are k-step 2 mt, the others 2 mt + 1
 #pragma unroll
-  for (int w = 0; w < LW; ++w) live[w] = __reduce_or_sync(kFull, live[w] << (g >> 2));
+  for (int w = 0; w < LW; ++w)
+    if (MARKS) live[w] = __reduce_or_sync(kFull, live[w] << (g >> 2));
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
 #pragma unroll
