@@ -959,9 +959,16 @@ void launch_fista_sparse_p(csd_handle* h, const csd::FistaParams& p) {
 // through the caches, alpha-ratio 1e-3 72 / 101 ms).
 int64_t dmma_voxels(const csd_handle* h) { return static_cast<int64_t>(h->K == 29 ? 80 : 56) * h->num_sms; }
 
-bool sparse_fista(const csd_handle* h, int64_t n_work) {
+// A fit of few iterations has no long tail, so DMMA slots lead from fewer voxels
+// where the iterates are dense (100 iterations, sparse warps / DMMA: order 6,
+// 6,000 voxels alpha 0.01 0.49 / 0.55 ms, 0.001 1.02 / 0.66; 9,000 voxels 0.62 /
+// 0.54, 1.34 / 0.66; order 4, 8,000 voxels 0.35 / 0.35, 0.50 / 0.35).
+bool short_fista(const csd::FistaParams& p) { return p.max_iter <= 2 * kSchedCap; }
+int64_t short_voxels(const csd_handle* h) { return static_cast<int64_t>(h->K == 29 ? 48 : 36) * h->num_sms; }
+
+bool sparse_fista(const csd_handle* h, const csd::FistaParams& p) {
   if (h->K == 145) return true;
-  return h->opt_shape == 0 && (h->K == 29 || h->K == 72) && n_work < dmma_voxels(h);
+  return h->opt_shape == 0 && (h->K == 29 || h->K == 72) && p.n_work < (short_fista(p) ? short_voxels(h) : dmma_voxels(h));
 }
 
 // A single pass on sparse warps or on DMMA slots, chosen by the alphas
@@ -970,7 +977,8 @@ bool sparse_fista(const csd_handle* h, int64_t n_work) {
 // the caller's order (slowest first by its own account, which the two passes
 // would not keep), and at order 6 for up to kChooseVoxels per SM in any order:
 // two passes cost a sparse alpha 0.14 ms there (8,300 voxels, alpha 0.01: 1.06
-// ms against 0.93 on sparse warps), the choice 0.01 ms.
+// ms against 0.93 on sparse warps), the choice 0.01 ms.  Fits of few iterations
+// choose from short_voxels() to dmma_voxels().
 // Fits of DifferentiableShore, N = 259, alpha_max about 0.33, sparse warps / DMMA
 // slots in ms by alpha:
 //   order 6             0.05       0.02       0.01       0.005      0.002      0.001
@@ -986,6 +994,7 @@ constexpr int64_t kChooseVoxels = 72;
 
 bool chosen_fista(const csd_handle* h, const csd::FistaParams& p) {
   if (h->opt_shape != 0 || (h->K != 29 && h->K != 72) || p.n_work_dev) return false;
+  if (short_fista(p)) return p.n_work < dmma_voxels(h);
   if (h->sched_off > 0 && p.list) return p.n_work < kSchedMinWaves * h->num_sms * 16 * 8;
   return h->K == 72 && p.n_work < kChooseVoxels * h->num_sms;
 }
@@ -996,7 +1005,8 @@ void choose_by_alpha(csd_handle* h, const csd::FistaParams& p, const unsigned lo
   auto* len = reinterpret_cast<unsigned long long*>(static_cast<char*>(h->schedCnt.p) +
                                                     kSchedSlotBytes * h->sched_slot + kSchedNnzAt) + 1;
   const double per_sm = static_cast<double>(p.n_work) / h->num_sms;
-  const double low = 3.6e-5 * per_sm * (1.0 + per_sm / 700.0), high = std::max(0.045, 17.0 / per_sm);
+  const double low = short_fista(p) ? 0.012 : 3.6e-5 * per_sm * (1.0 + per_sm / 700.0);
+  const double high = std::max(0.045, 17.0 / per_sm);
   csd::k_choose_by_alpha<<<1, 1024, 0, h->stream>>>(p, h->K, h->Kp, low, high, len + 1, len);
   CSD_LAUNCH();
   n = len;
@@ -1684,7 +1694,7 @@ void launch_fista(csd_handle* h, int MT, const csd::FistaParams& p) {
     CSD_LAUNCH();
     return;
   }
-  if (sparse_fista(h, p.n_work)) {
+  if (sparse_fista(h, p)) {
     launch_fista_sparse(h, p);
     return;
   }

@@ -46,6 +46,24 @@ def test_dense_fits_match_the_dmma_kernel_bit_for_bit(order, v, kw):
         np.testing.assert_array_equal(chosen[k], dmma[k])
 
 
+@pytest.mark.parametrize("order,v", [(4, 7103), (4, 7104), (4, 11839), (4, 11840), (6, 5327), (6, 5328), (6, 8287),
+                                     (6, 8288)])
+@pytest.mark.parametrize("max_iter", [20, 160, 161])
+@pytest.mark.parametrize("alpha", [0.0005, 0.02])
+def test_short_fits_match_the_dmma_kernel_bit_for_bit(order, v, max_iter, alpha):
+    from cs_dmri_b200 import _abi
+    ph, data, mask = tiled(v)
+    kw = dict(radial_order=order, alpha_mode="fixed", alpha=alpha, max_iter=max_iter)
+    chosen = fit(ph, data, mask, **kw)
+    _abi.set_option(_abi.OPT_FISTA_SHAPE, 12)
+    try:
+        dmma = fit(ph, data, mask, **kw)
+    finally:
+        _abi.set_option(_abi.OPT_FISTA_SHAPE, 0)
+    for k in KEYS:
+        np.testing.assert_array_equal(chosen[k], dmma[k])
+
+
 @pytest.mark.parametrize("order,v", [(4, 20000), (4, 25001), (4, 25056), (6, 15000), (6, 20000), (6, 76000)])
 def test_the_second_pass_follows_the_density(order, v):
     ph, data, mask = tiled(v)
