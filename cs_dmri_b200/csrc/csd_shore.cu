@@ -497,7 +497,7 @@ void ensure_setup(csd_handle* h, const HostGtab& g, int radial_order, double zet
     const int MT = Kp / 8, KT = Kp / 4;
     h->gfrag.ensure(sizeof(double) * MT * KT * 32);
     h->scal.ensure(sizeof(double) * 4);
-    h->ok.ensure(sizeof(int) * 4);
+    h->ok.ensure(sizeof(csd::CholeskyResult));
     // 4 pi^2 tau in the reference's evaluation order (src/qspace.rs:384-385).
     const double qdenom = 4.0 * kPi * kPi * g.tau;
     const long long nk = static_cast<long long>(N) * K;
@@ -567,13 +567,13 @@ void ensure_setup(csd_handle* h, const HostGtab& g, int radial_order, double zet
       const size_t csm = sizeof(double) * static_cast<size_t>(K) * K;
       CSD_CUDA(cudaFuncSetAttribute(csd::k_cholesky, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     static_cast<int>(csm)));
-      csd::k_cholesky<<<1, 256, csm, st>>>(h->A.as<double>(), K, Kp, h->ok.as<int>(), h->scal.as<double>() + 2);
+      csd::k_cholesky<<<1, 256, csm, st>>>(h->A.as<double>(), K, Kp, h->ok.as<csd::CholeskyResult>());
       CSD_LAUNCH();
-      int okv = 0;
-      CSD_CUDA(cudaMemcpyAsync(&okv, h->ok.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-      CSD_CUDA(cudaMemcpyAsync(&h->chol_growth, h->scal.as<double>() + 2, sizeof(double), cudaMemcpyDeviceToHost, st));
+      csd::CholeskyResult res{};
+      CSD_CUDA(cudaMemcpyAsync(&res, h->ok.p, sizeof res, cudaMemcpyDeviceToHost, st));
       CSD_CUDA(cudaStreamSynchronize(st));
-      if (!okv) throw Error{CSD_ERR_NUMERICAL, "normal-equations matrix should be PD"};
+      h->chol_growth = res.growth;
+      if (!res.ok) throw Error{CSD_ERR_NUMERICAL, "normal-equations matrix should be PD"};
       h->chol_key = ck;
       h->chol_valid = true;
       // P^T = rows H^-1 m_n of the design rows m_n, by the factor's solves:
@@ -640,12 +640,12 @@ void ensure_icls_setup(csd_handle* h, int radial_order, double zeta, double eps)
   const size_t csm = sizeof(double) * static_cast<size_t>(K) * K;
   CSD_CUDA(cudaFuncSetAttribute(csd::k_cholesky, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(csm)));
-  csd::k_cholesky<<<1, 256, csm, st>>>(h->Le.as<double>(), K, Kp, h->ok.as<int>(), nullptr);
+  csd::k_cholesky<<<1, 256, csm, st>>>(h->Le.as<double>(), K, Kp, h->ok.as<csd::CholeskyResult>());
   CSD_LAUNCH();
-  int okv = 0;
-  CSD_CUDA(cudaMemcpyAsync(&okv, h->ok.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+  csd::CholeskyResult res{};
+  CSD_CUDA(cudaMemcpyAsync(&res, h->ok.p, sizeof res, cudaMemcpyDeviceToHost, st));
   CSD_CUDA(cudaStreamSynchronize(st));
-  if (!okv) throw Error{CSD_ERR_NUMERICAL, "H^T H + eps I must be positive definite"};
+  if (!res.ok) throw Error{CSD_ERR_NUMERICAL, "H^T H + eps I must be positive definite"};
   h->Wi.ensure(sizeof(double) * static_cast<size_t>(K) * m_pad);
   csd::k_icls_w<<<(m_pad + 127) / 128, 128, 0, st>>>(h->Le.as<double>(), K, Kp, h->Cmat.as<double>(), m, m_pad,
                                                       h->Wi.as<double>());

@@ -162,14 +162,17 @@ __global__ void k_lipschitz(const double* __restrict__ G, int Kp, int N, int max
   }
 }
 
+struct CholeskyResult {
+  int ok, pad;
+  double growth;  // max_j A_jj / l_jj^2
+};
+
 // In-place right-looking Cholesky A = L L^T of the leading K x K block of a
-// Kp x Kp matrix, one CTA.  Writes 0 to *ok_out if A is not positive definite
-// (the reference panics there, src/solver/tikhonov.rs:44).  The accumulation
+// Kp x Kp matrix, one CTA.  res->ok is 0 if A is not positive definite (the
+// reference panics there, src/solver/tikhonov.rs:44).  The accumulation
 // order of every entry is the left-looking order k = 0, 1, ..., so results
-// match a sequential LL^T factorisation.  max_j A_jj / l_jj^2 goes to *growth_out
-// (nullable).
-__global__ void k_cholesky(double* __restrict__ A, int K, int Kp, int* __restrict__ ok_out,
-                           double* __restrict__ growth_out) {
+// match a sequential LL^T factorisation.
+__global__ void k_cholesky(double* __restrict__ A, int K, int Kp, CholeskyResult* __restrict__ res) {
   extern __shared__ double sA[];
   __shared__ int s_ok;
   __shared__ unsigned long long s_growth;
@@ -198,19 +201,19 @@ __global__ void k_cholesky(double* __restrict__ A, int K, int Kp, int* __restric
     }
     __syncthreads();
   }
-  if (growth_out) {
-    for (int j = tid; j < K; j += nt) {
-      const double l = sA[j * K + j], g = A[j * Kp + j] / (l * l);
-      atomicMax(&s_growth, static_cast<unsigned long long>(__double_as_longlong(g > 0.0 ? g : 0.0)));  // orders as its bits
-    }
-    __syncthreads();
-    if (tid == 0) *growth_out = __longlong_as_double(static_cast<long long>(s_growth));
+  for (int j = tid; j < K; j += nt) {
+    const double l = sA[j * K + j], g = A[j * Kp + j] / (l * l);
+    atomicMax(&s_growth, static_cast<unsigned long long>(__double_as_longlong(g > 0.0 ? g : 0.0)));  // orders as its bits
   }
+  __syncthreads();
   for (int i = tid; i < Kp * Kp; i += nt) {
     const int r = i / Kp, c = i % Kp;
     A[i] = (r < K && c < K && c <= r) ? sA[r * K + c] : 0.0;
   }
-  if (tid == 0) *ok_out = s_ok;
+  if (tid == 0) {
+    res->ok = s_ok;
+    res->growth = __longlong_as_double(static_cast<long long>(s_growth));
+  }
 }
 
 // Pack the symmetric Gram matrix into m8n8k4 DMMA A-operand tiles:
