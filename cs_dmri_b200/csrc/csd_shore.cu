@@ -560,6 +560,7 @@ void ensure_setup(csd_handle* h, const HostGtab& g, int radial_order, double zet
     uint64_t ck = fnv1a(key, &lambda_n, sizeof lambda_n);
     ck = fnv1a(ck, &lambda_l, sizeof lambda_l);
     if (!(h->chol_valid && h->chol_key == ck)) {
+      h->chol_valid = h->pfrag_valid = h->l2mat_valid = false;  // A is overwritten, also by a factor that fails
       csd::k_gram<<<(Kp * Kp + 255) / 256, 256, 0, st>>>(h->M.as<double>(), N, K, Kp, radial_order,
                                                         lambda_n, lambda_l, h->G.as<double>(),
                                                         h->A.as<double>());
@@ -579,7 +580,6 @@ void ensure_setup(csd_handle* h, const HostGtab& g, int radial_order, double zet
       // P^T = rows H^-1 m_n of the design rows m_n, by the factor's solves:
       // packed like M^T for the right-hand-side kernel, or as it stands, with
       // the rows of H^-1 from the same launch, for the apply kernel
-      h->pfrag_valid = h->l2mat_valid = false;
       const bool apply = !h->dmma_rhs && l2_product_exact(h) && apply_dmma_fits(h, N);
       if (h->dmma_rhs || apply) {
         const size_t rows = static_cast<size_t>(N) + (apply ? K : 0);

@@ -93,3 +93,14 @@ def test_host_and_device_paths_share_the_l2_reference(order, lam, slack):
     dev, _ = shore_fit_device(torch.from_numpy(np.ascontiguousarray(data)).cuda(), torch.from_numpy(mask).cuda(),
                               ph.bvals, ph.bvecs, **kw)
     np.testing.assert_array_equal(host, dev.cpu().numpy())
+
+
+@pytest.mark.parametrize("lam", [1e-9, 0.05])  # by the substitutions, by the product
+def test_a_refused_factor_leaves_no_trace(lam):
+    """150 directions cannot determine 145 coefficients without a weight: the
+    factor fails, and the fit with the earlier weight is what it was."""
+    bvals, bvecs, _, _, s = system(8, 150, lam)
+    want = gpu_fit(8, bvals, bvecs, s, lam)
+    with pytest.raises(Exception, match="should be PD"):
+        gpu_fit(8, bvals, bvecs, s, 0.0)
+    np.testing.assert_array_equal(gpu_fit(8, bvals, bvecs, s, lam), want)
