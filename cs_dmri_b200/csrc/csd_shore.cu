@@ -618,6 +618,7 @@ void ensure_icls_setup(csd_handle* h, int radial_order, double zeta, double eps)
   cudaStream_t st = h->stream;
   uint64_t key = fnv1a(h->setup_key, &eps, sizeof eps);
   if (h->icls_valid && h->icls_key == key) return;
+  h->icls_valid = false;  // the buffers are overwritten, also by a factor that fails
   const int K = h->K, Kp = h->Kp;
   const std::vector<double> dirs = hemisphere_directions();
   const int m = static_cast<int>(dirs.size() / 3);
