@@ -647,7 +647,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_path_dmma(PathParams pp, int par
   double thr[2] = {INFINITY, INFINITY};
   bool need[2] = {true, true};
   bool exhausted = false;
-  unsigned executed = 0;
+  unsigned executed = 0, ksteps = 0;
   unsigned live[1] = {kFull};
   auto columns = [&](bool f0, bool f1) {  // the slots whose lanes set a flag
     const unsigned n0 = __ballot_sync(kFull, lane < 4 && f0), n1 = __ballot_sync(kFull, lane < 4 && f1);
@@ -731,7 +731,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_path_dmma(PathParams pp, int par
     double mom[2], dx2[2], xn2[2];
 #pragma unroll
     for (int j = 0; j < 2; ++j) mom[j] = vid[j] >= 0 ? p.mom[it[j]] : 0.0;
-    dmma_fista_step<MT, NONNEG>(sG, ybuf, bbuf, live, x, mom, thr, c, lane, dx2, xn2);
+    ksteps += dmma_fista_step<MT, NONNEG>(sG, ybuf, bbuf, live, x, mom, thr, c, lane, dx2, xn2);
 
     // ---- per-voxel stopping rule (fista.rs:115-127)
     bool conv[2] = {false, false}, fin[2] = {false, false};
@@ -808,6 +808,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_path_dmma(PathParams pp, int par
     for (int o = 16; o > 0; o >>= 1) executed += __shfl_xor_sync(kFull, executed, o);
     if (lane == 0) atomicAdd(p.iter_total, static_cast<unsigned long long>(executed));
   }
+  if (p.kstep_total && lane == 0) atomicAdd(p.kstep_total, static_cast<unsigned long long>(ksteps));
 }
 
 }  // namespace csd

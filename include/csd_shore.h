@@ -235,7 +235,7 @@ typedef struct csd_fit_timing {
   float ms_total;       /* device time from first to last kernel */
   int32_t launches;     /* kernels launched by the fit */
   float ms_solve_kernel;/* duration of the dominant solve kernel alone */
-  double tensor_flops;  /* FP64 tensor-core FLOPs the FISTA launches executed (0 where sparse warps serve) */
+  double tensor_flops;  /* FP64 tensor-core FLOPs the FISTA launches executed (sparse warps execute none) */
   float ms_mixed_kernel;/* the mixed-precision FISTA kernel alone (0 in FP64) */
   double int8_tensor_ops;      /* int8 tensor-core ops it issued (2 per MAC) */
   uint64_t fp64_rerun_voxels;  /* voxels the stop-decision guard re-ran in FP64 */
