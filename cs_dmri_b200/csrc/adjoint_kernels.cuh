@@ -262,8 +262,7 @@ __global__ void k_identity_rows(double* __restrict__ I, int K, int Kp) {
 // through a ring of kApplyPf fragments, refilled in place as their DMMAs are
 // issued (a register move would wait for the load still in flight).  Every
 // tile accumulates its k-steps in increasing order: one FMA chain in index
-// order, as k_rhs.  With `add` (laid out as out, which it may be)
-// the output is add + sign A in.
+// order, as k_rhs.
 //
 // Chunks of row tiles: a matrix larger than one CTA's shared memory (the
 // order-8 ODF, adjoint and design products take 300-420 KB) ran on plain FMAs,
@@ -278,7 +277,7 @@ template <class TIn>
 __global__ void __launch_bounds__(32 * kApplyWarps, 1)
     k_apply_dmma(const double* __restrict__ At, int lda, int rows, int cols, int mt_chunk, const TIn* __restrict__ in,
                  int64_t ldin, const int64_t* __restrict__ idx, int64_t V, double* __restrict__ out,
-                 float* __restrict__ out32, int64_t ldout, int rows_out, const double* add, double sign) {
+                 float* __restrict__ out32, int64_t ldout, int rows_out) {
   extern __shared__ __align__(16) double sA[];
   const int mt_first = blockIdx.y * mt_chunk;
   const int MT = min(mt_chunk, (rows_out + 7) / 8 - mt_first), KT = (cols + 3) / 4;
@@ -344,9 +343,8 @@ __global__ void __launch_bounds__(32 * kApplyWarps, 1)
         for (int e = 0; e < 2; ++e) {
           const int64_t vv = 8 * grp + 2 * q + e;
           if (vv < V) {
-            const double o = add ? fma(sign, d[j][e], add[vv * ldout + r]) : d[j][e];
-            if (out) out[vv * ldout + r] = o;
-            if (out32) out32[vv * ldout + r] = static_cast<float>(o);
+            if (out) out[vv * ldout + r] = d[j][e];
+            if (out32) out32[vv * ldout + r] = static_cast<float>(d[j][e]);
           }
         }
       }

@@ -1719,8 +1719,7 @@ bool apply_dmma_fits(const csd_handle* h, int cols) {
 // At with row stride lda), rows_out >= rows outputs (zeros past rows).
 template <class TIn>
 void launch_apply_dmma(csd_handle* h, const double* At, int lda, int rows, int cols, const TIn* in, int64_t ldin,
-                       const int64_t* idx, int64_t V, double* out, float* out32, int64_t ldout, int rows_out,
-                       const double* add = nullptr, double sign = 1.0) {
+                       const int64_t* idx, int64_t V, double* out, float* out32, int64_t ldout, int rows_out) {
   constexpr int W = csd::kApplyWarps;
   const size_t tile = sizeof(double) * 32 * static_cast<size_t>((cols + 3) / 4);
   const int MT = (rows_out + 7) / 8;
@@ -1738,7 +1737,7 @@ void launch_apply_dmma(csd_handle* h, const double* At, int lda, int rows, int c
   auto* kern = csd::k_apply_dmma<TIn>;
   CSD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
   kern<<<dim3(static_cast<unsigned>(bx), static_cast<unsigned>(chunks)), 32 * W, smem, h->stream>>>(
-      At, lda, rows, cols, mt_chunk, in, ldin, idx, V, out, out32, ldout, rows_out, add, sign);
+      At, lda, rows, cols, mt_chunk, in, ldin, idx, V, out, out32, ldout, rows_out);
   CSD_LAUNCH();
 }
 
