@@ -7,12 +7,14 @@
 //   PathL2Anchored  same path, keep the first (largest-alpha) point whose
 //                   RSS <= (1 + slack) RSS_L2, else the point of minimum RSS
 // with alpha_max = ||M^T s||_inf / n and the zero result for alpha_max == 0.
-// The path is walked one point at a time over the whole volume: each point is
-// one FISTA launch over the voxels still in play, warm-started in place from
-// the previous point (fista.rs:164-178), then one residual pass and the
-// selection update below.  Under PathL2Anchored a voxel leaves the work list
-// as soon as it is selected: the later points of its path cannot change the
-// result, so they are not computed.
+// The FP64 fits of radial orders 4, 6 and 8 walk each voxel's path on its own
+// slot (k_path_sparse, k_path_dmma); they share path_alpha and path_better with
+// the walk below, which serves order 2, the mixed precision and a forced kernel
+// shape: one point at a time over the whole volume, each point one FISTA launch
+// over the voxels still in play, warm-started in place from the previous point
+// (fista.rs:164-178), then one residual pass and the selection update.  Under
+// PathL2Anchored a voxel leaves the work list as soon as it is selected: the
+// later points of its path cannot change the result, so they are not computed.
 #pragma once
 
 #include <cstdint>
@@ -39,18 +41,41 @@ __global__ void k_alpha_ratio(const double* __restrict__ amax, int64_t V, double
   alpha[v] = amax[v] * ratio;
 }
 
-// Point i of log_path(alpha_max_v, n, eps) (src/solver/alpha.rs:57-69) for
-// the voxels of `list`.
+// Point i of log_path(alpha_max, n, eps) (src/solver/alpha.rs:57-69).
+__device__ __forceinline__ double path_alpha(double amax, int i, int n, double eps) {
+  const double lmax = log(amax), lmin = log(amax * eps);
+  const double t = static_cast<double>(i) / static_cast<double>(n - 1);
+  return exp(lmax + t * (lmin - lmax));
+}
+
+// Selection at one path point: PathBic keeps the lowest BIC (bic_argmin,
+// alpha.rs:107-128), PathL2Anchored the lowest RSS until one is within the
+// slack of the Tikhonov fit's, which ends the path (l2_anchored_argmax,
+// alpha.rs:140-165).
+__device__ __forceinline__ bool path_better(int mode, int N, int nnz, double rss, double rss_limit, double& best,
+                                            bool& last) {
+  if (mode == 2) {
+    const double n = static_cast<double>(N);
+    const double bic = n * log(fmax(rss, 2.2250738585072014e-308) / n) + log(n) * static_cast<double>(nnz);
+    if (!(bic < best)) return false;
+    best = bic;
+    return true;
+  }
+  const bool within = rss <= rss_limit;
+  last = last || within;
+  if (!within && !(rss < best)) return false;
+  best = rss;
+  return true;
+}
+
+// The alphas of point i for the voxels of `list`.
 __global__ void k_path_alpha(const double* __restrict__ amax, const int64_t* __restrict__ list,
                              int64_t n_work, int i, int n, double eps,
                              double* __restrict__ alpha) {
   const int64_t w = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (w >= n_work) return;
   const int64_t v = list[w];
-  const double lmax = log(amax[v]);
-  const double lmin = log(amax[v] * eps);
-  const double t = static_cast<double>(i) / static_cast<double>(n - 1);
-  alpha[v] = exp(lmax + t * (lmin - lmax));
+  alpha[v] = path_alpha(amax[v], i, n, eps);
 }
 
 struct PathState {
@@ -66,9 +91,8 @@ struct PathState {
   int8_t* copy_code;   // V: 0 none, 1 -> Xsel, 2 -> Xfb (this point)
 };
 
-// Selection update after path point `i` for the voxels of `list`.
-// mode 2 = PathBic (bic_argmin, alpha.rs:107-128),
-// mode 3 = PathL2Anchored (l2_anchored_argmax, alpha.rs:140-165).
+// Selection update after path point `i` for the voxels of `list` (mode 2 =
+// PathBic, mode 3 = PathL2Anchored).
 __global__ void k_path_update(int mode, const int64_t* __restrict__ list, int64_t n_work, int N,
                               const double* __restrict__ resid, const int* __restrict__ nnz,
                               const double* __restrict__ alpha, const uint32_t* __restrict__ iters,
@@ -79,33 +103,19 @@ __global__ void k_path_update(int mode, const int64_t* __restrict__ list, int64_
   const int64_t v = list[w];
   const double rss = resid[v] * resid[v];
   int8_t code = 0;
-  if (mode == 2) {
-    const double n = static_cast<double>(N);
-    const double rc = fmax(rss, 2.2250738585072014e-308);
-    const double b = n * log(rc / n) + log(n) * static_cast<double>(nnz[v]);
-    if (b < s.best[v]) {
-      s.best[v] = b;
-      s.alpha_sel[v] = alpha[v];
-      s.it_sel[v] = iters[v];
-      s.conv_sel[v] = conv[v];
-      code = 1;
-    }
-  } else {
-    const double thr = (1.0 + slack) * rss_l2[v];
-    if (rss <= thr) {
-      s.selected[v] = 1;
-      s.active[v] = 0;
-      s.alpha_sel[v] = alpha[v];
-      s.it_sel[v] = iters[v];
-      s.conv_sel[v] = conv[v];
-      code = 1;
-    } else if (rss < s.best[v]) {
-      s.best[v] = rss;
-      s.alpha_fb[v] = alpha[v];
-      s.it_fb[v] = iters[v];
-      s.conv_fb[v] = conv[v];
-      code = 2;
-    }
+  bool last = false;
+  double best = s.best[v];
+  if (path_better(mode, N, nnz[v], rss, mode == 3 ? (1.0 + slack) * rss_l2[v] : 0.0, best, last)) {
+    s.best[v] = best;
+    const bool chosen = mode == 2 || last;  // else PathL2Anchored's fallback, the lowest RSS so far
+    code = chosen ? 1 : 2;
+    (chosen ? s.alpha_sel : s.alpha_fb)[v] = alpha[v];
+    (chosen ? s.it_sel : s.it_fb)[v] = iters[v];
+    (chosen ? s.conv_sel : s.conv_fb)[v] = conv[v];
+  }
+  if (last) {
+    s.selected[v] = 1;
+    s.active[v] = 0;
   }
   s.copy_code[v] = code;
 }

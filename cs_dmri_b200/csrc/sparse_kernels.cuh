@@ -393,33 +393,6 @@ struct PathParams {
   int resume;            // take the parked voxels (*n_park of them) instead of 0 .. n_work-1
 };
 
-// Point i of log_path(alpha_max, n, eps) (src/solver/alpha.rs:57-69).
-__device__ __forceinline__ double path_alpha(double amax, int i, int n, double eps) {
-  const double lmax = log(amax), lmin = log(amax * eps);
-  const double t = static_cast<double>(i) / static_cast<double>(n - 1);
-  return exp(lmax + t * (lmin - lmax));
-}
-
-// Selection at one path point: PathBic keeps the lowest BIC (bic_argmin,
-// alpha.rs:107-128), PathL2Anchored the lowest RSS until one is within the
-// slack of the Tikhonov fit's, which ends the path (l2_anchored_argmax,
-// alpha.rs:140-165).
-__device__ __forceinline__ bool path_better(int mode, int N, int nnz, double rss, double rss_limit, double& best,
-                                            bool& last) {
-  if (mode == 2) {
-    const double n = static_cast<double>(N);
-    const double bic = n * log(fmax(rss, 2.2250738585072014e-308) / n) + log(n) * static_cast<double>(nnz);
-    if (!(bic < best)) return false;
-    best = bic;
-    return true;
-  }
-  const bool within = rss <= rss_limit;
-  last = last || within;
-  if (!within && !(rss < best)) return false;
-  best = rss;
-  return true;
-}
-
 // ||s - M c||^2 of one voxel on a warp, c sparse (listed in increasing row as
 // values, every P-th double, and rows): four samples a lane and
 // four coefficients at a time, so 16 loads are in flight; the columns of M are
