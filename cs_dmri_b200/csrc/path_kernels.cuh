@@ -136,14 +136,15 @@ __global__ void k_path_copy(const int64_t* __restrict__ list, int64_t n_work, in
 }
 
 // PathL2Anchored voxels that never met the slack bound take their
-// minimum-RSS point.
+// minimum-RSS point; one without any (a residual that is not finite) keeps the
+// zero result.
 __global__ void k_path_finalize(int64_t V, int Kp, const uint8_t* __restrict__ zero, PathState s,
                                 const double* __restrict__ Xfb, double* __restrict__ Xsel) {
   const int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (e >= V * Kp) return;
   const int64_t v = e / Kp;
   const int k = static_cast<int>(e % Kp);
-  if (zero[v] || s.selected[v]) return;
+  if (zero[v] || s.selected[v] || !(s.best[v] < INFINITY)) return;
   Xsel[v * Kp + k] = Xfb[v * Kp + k];
   if (k == 0) {
     s.alpha_sel[v] = s.alpha_fb[v];

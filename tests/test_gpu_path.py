@@ -74,3 +74,18 @@ def test_the_path_on_dmma_slots_counts_its_tensor_operations():
     out = fit(ph, data, mask, radial_order=6, alpha_mode="l2-anchored", path_n_alphas=7)
     dense = 2.0 * 72 * 72 * out["total_iterations"]  # live k-steps only, and slots left empty
     assert 0.1 * dense < _abi.last_timing(0).tensor_flops < 1.5 * dense
+
+
+@pytest.mark.parametrize("order", [2, 6])
+def test_a_path_without_a_finite_residual_gives_zero(order):
+    """The walk and the fused path alike; the walk's scratch holds another fit's
+    fallback points from the call before."""
+    ph, data, mask = tiled(96)
+    kw = dict(radial_order=order, alpha_mode="l2-anchored", path_n_alphas=5, slack=0.0)
+    run = walked if order == 6 else fit
+    run(ph, data, mask, **kw)
+    bad = data.copy()
+    bad[40, 0, 0, 9] = np.inf
+    for out in (run(ph, bad, mask, **kw), fit(ph, bad, mask, **kw)):
+        assert not out["coef64"][40].any() and out["alpha"].ravel()[40] == 0.0
+        assert out["iterations"].ravel()[40] == 0 and out["converged"].ravel()[40]
