@@ -79,7 +79,7 @@ def parse():
     ap.add_argument("--cpu-seconds", type=float, default=12.0, help="target length of the CPU sample")
     ap.add_argument("--no-cpu", action="store_true", help="skip the CPU baseline leg")
     ap.add_argument("--profile-case", choices=["graddev2k", "graddev2k-mixed", "diff50k", "peaks108k", "fista125k",
-                                               "kkt64k", "icls64k", "tikhonov64k"],
+                                               "fista4k", "path30k", "kkt64k", "icls64k", "tikhonov64k"],
                     help="run one small profiling workload instead of the benchmark")
     ap.add_argument("--workload", choices=["brain300k", "grid64k"], default="brain300k",
                     help="brain300k: the benchmark volume; grid64k: 40^3 fully masked (profiling case)")
@@ -980,9 +980,11 @@ def case_peaks108k() -> None:
 
 def case_fista125k() -> None:
     """A fixed-alpha fit of a 50^3 phantom (125,000 voxels, K = 72) through the
-    device entry point: enough voxels per FISTA slot for the two-pass
-    schedule (pass 1 to iteration 80, bucket sort, pass 2).  A first fit
-    (gradient-table set-up, autotuning) runs outside the NVTX range."""
+    device entry point on the DMMA kernel, with the two-pass schedule (pass 1
+    to iteration 80, bucket sort, pass 2) as a brain-sized volume runs it: the
+    shape is given, because the library's own choice at this size puts the
+    second pass on sparse warps.  A first fit (gradient-table set-up,
+    autotuning) runs outside the NVTX range."""
     import torch
 
     from cs_dmri_b200 import _abi
@@ -992,6 +994,7 @@ def case_fista125k() -> None:
     d = torch.from_numpy(ph.data).cuda()
     m = torch.from_numpy(ph.mask).cuda()
     kw = dict(big_delta=ph.big_delta, small_delta=ph.small_delta, alpha_mode="fixed", alpha=0.01)
+    _abi.set_option(_abi.OPT_FISTA_SHAPE, 16)
     shore_fit_device(d, m, ph.bvals, ph.bvecs, **kw)
     torch.cuda.synchronize()
     torch.cuda.nvtx.range_push("fista125k")
@@ -1002,12 +1005,41 @@ def case_fista125k() -> None:
     print(f"fista125k: solve {t.ms_solve_kernel:.3f} ms, parked {t.fista_parked} of {int(ph.mask.sum())} voxels")
 
 
+def _case_phantom(name: str, shape, **fit_kw) -> None:
+    """One fit of a phantom of the shape through the device entry point after a
+    set-up fit of the same kind."""
+    import torch
+
+    from cs_dmri_b200 import _abi
+    from cs_dmri_b200._core import shore_fit_device
+    from cs_dmri_b200.phantom import make_phantom
+    ph = make_phantom(shape, seed=6)
+    d = torch.from_numpy(ph.data).cuda()
+    m = torch.from_numpy(ph.mask).cuda()
+    kw = dict(big_delta=ph.big_delta, small_delta=ph.small_delta, **fit_kw)
+    for _ in range(2):
+        shore_fit_device(d, m, ph.bvals, ph.bvecs, **kw)
+    torch.cuda.synchronize()
+    t = _abi.last_timing(0)
+    print(f"{name}: solve kernel {t.ms_solve_kernel:.3f} ms, total {t.ms_total:.3f} ms")
+
+
+def case_fista4k() -> None:
+    """A fixed-alpha fit of 4,000 voxels: k_fista_sparse, one voxel per warp."""
+    _case_phantom("fista4k", (20, 20, 10), alpha_mode="fixed", alpha=0.01)
+
+
+def case_path30k() -> None:
+    """The L2-anchored path on 30,720 voxels: k_path_dmma, then k_path_sparse on
+    the voxels that it parks."""
+    _case_phantom("path30k", (32, 32, 30), alpha_mode="l2-anchored")
+
+
 def case_kkt64k() -> None:
     """The converged-optimum fit (precision "mixed-kkt") of the 40^3 phantom
     (64,000 voxels, K = 72) through the device entry point, 32 support
-    iterations: one launch each of k_fista_tf32 and the two k_l1_polish passes
-    per fit.  A first fit (set-up) runs before the
-    measured one."""
+    iterations: k_fista_tf32, then k_l1_polish_half and the k_l1_polish passes
+    per fit.  A first fit (set-up) runs before the measured one."""
     import torch
 
     from cs_dmri_b200 import _abi
@@ -1048,7 +1080,7 @@ def _case_grid64k(name: str, **fit_kw) -> None:
 
 
 def case_icls64k() -> None:
-    """The amplitude-positivity QP (k_icls) on the 40^3 phantom."""
+    """The amplitude-positivity QP (k_icls_gram) on the 40^3 phantom."""
     _case_grid64k("icls64k", regularization="nonneg")
 
 
@@ -1059,8 +1091,8 @@ def case_tikhonov64k() -> None:
 
 
 PROFILE_CASES = {"graddev2k": case_graddev2k, "graddev2k-mixed": case_graddev2k_mixed, "diff50k": case_diff50k, "peaks108k": case_peaks108k,
-                 "fista125k": case_fista125k, "kkt64k": case_kkt64k, "icls64k": case_icls64k,
-                 "tikhonov64k": case_tikhonov64k}
+                 "fista125k": case_fista125k, "fista4k": case_fista4k, "path30k": case_path30k,
+                 "kkt64k": case_kkt64k, "icls64k": case_icls64k, "tikhonov64k": case_tikhonov64k}
 
 
 def launch_ranks(args) -> int:

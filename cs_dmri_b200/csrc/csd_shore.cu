@@ -1101,7 +1101,11 @@ void launch_path_dmma_p(csd_handle* h, const csd::PathParams& p, int park_at) {
 // point: L2-anchored 4,000 voxels 18.7 / 12.9 / 18.1 ms, 30,211 voxels (N =
 // 181) 44.8 / 53.3 / 59.9 ms, 148,877 voxels 159 / 247 / 184 ms; path-BIC
 // 8,000 voxels 35.6 / 34.4 / 41.8 ms, 64,000 voxels 130 / 205 / 207 ms; order
-// 4, 64,000 voxels 22 / 36 / 40 ms.
+// 4, 64,000 voxels 22 / 36 / 40 ms.  On the sparse kernel one / two voxels per warp
+// (order 8, L2-anchored): 600 voxels 8.7 / 14.0 ms, 2,400 17.1 / 20.8, 4,000 27.1 /
+// 26.4, 15,000 86.8 / 79.3 (one is taken throughout); one CTA of 16 warps per SM at
+// order 4, without the spills that two are held to 64 registers by, 2,400 voxels
+// 3.6 -> 2.4 ms, 9,000 6.7 -> 6.2 (two are taken).
 constexpr int kPathDmmaVoxels = 64;
 constexpr int kPathParkAt = 4;  // active slots of a warp at which it parks them: 0 47.6, 2 45.7, 4 44.8, 6 47.2 ms
 

@@ -24,8 +24,9 @@
 //      its entries non-zero at order 8, so the listed columns alone are added
 //      (SparseFista), with no barrier in an iteration.
 //
-// What bounds it: latency, one voxel at a time per SM (two CTAs at order 6; G_v
-// takes 169 KB at order 8).  SM cycles per voxel at order 8, reference rule,
+// What bounds it: latency, one voxel at a time per SM (the grid has one CTA per SM
+// at both orders; G_v takes 169 KB at order 8 and 42 KB at order 6, where a second
+// CTA would fit).  SM cycles per voxel at order 8, reference rule,
 // ~145 iterations: Gram step 112 k (~50 k of it the DMMA pipe's floor), Lanczos
 // 155 k (40 steps of ~3.4 k and ~18 k for the tridiagonal's eigenvalue; one
 // thread per row of the product and a Sturm count with a division a step took

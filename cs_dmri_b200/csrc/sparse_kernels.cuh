@@ -13,12 +13,14 @@
 // order 6: 100 wavefronts of 128 B a voxel-iteration, 85 % of the pipe's
 // rate; two per warp read each column of their common list once: 72, at 65 %
 // with the issue slots at 63 %); for a few voxels the latency of one
-// iteration, 0.5-0.6 us against the 1.25-2 us of a DMMA warp.  An SM partition
-// takes 32 B a cycle from shared memory, broadcasts included, so a column
-// costs its warp 18 cycles at order 6 and 36 at order 8 besides 12 for its
-// list entry.  Volume fits, N = 259, against the DMMA kernel alone: 108 voxels
-// 1.64 -> 0.42 ms, 4,000 voxels 3.55 -> 0.84 ms, 32,000 voxels at order 8
-// 11.4 -> 3.5 ms (with the residual pass that no output reads dropped there).
+// iteration, 0.3 us for a lone warp and 0.5-0.6 us beside fifteen others,
+// against the 1.25-4 us of a DMMA warp.  An SM partition takes 32 B a cycle from
+// shared memory, broadcasts included, so a column costs its warp 18 cycles at
+// order 6 and 36 at order 8 besides 12 for its list entry: dense iterates belong
+// on DMMA slots (PassChoice, k_choose_by_alpha).  Volume fits, N = 259, alpha
+// 0.01, against the DMMA kernel alone: 108 voxels 1.64 -> 0.42 ms, 4,000 voxels
+// 3.55 -> 0.84 ms, 32,000 voxels at order 8 11.4 -> 3.5 ms (with the residual pass
+// that no output reads dropped there).
 #pragma once
 
 #include <cstdint>

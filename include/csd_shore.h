@@ -266,9 +266,10 @@ int csd_last_timing(const csd_handle* h, csd_fit_timing* out);
 
 /* Tuning options of a handle (they never change a result's meaning):
  *   CSD_OPT_FISTA_SHAPE     FP64 FISTA kernel: 0 = the library's choice by
- *                           size and radial order (default: sparse warps,
- *                           the DMMA kernel with the per-table autotuned
- *                           shape, or both in turn; alpha paths fused), 12
+ *                           size, radial order and density of the iterates
+ *                           (default: sparse warps, the DMMA kernel with the
+ *                           per-table autotuned shape, or both in turn;
+ *                           alpha paths fused), 12
  *                           or 16 warps per CTA of the DMMA kernel, 1 = the
  *                           register kernel; every shape computes the same
  *                           iterates
