@@ -269,8 +269,8 @@ int csd_last_timing(const csd_handle* h, csd_fit_timing* out);
  *                           size, radial order and density of the iterates
  *                           (default: sparse warps, the DMMA kernel with the
  *                           per-table autotuned shape, or both in turn;
- *                           alpha paths fused), 12
- *                           or 16 warps per CTA of the DMMA kernel, 1 = the
+ *                           alpha paths fused), 12 or 16 = the DMMA kernel
+ *                           with up to that many warps per CTA, 1 = the
  *                           register kernel; every shape computes the same
  *                           iterates
  *   CSD_OPT_FISTA_SCHEDULE  0 = single-pass FISTA; 1 = the two-pass
